@@ -64,6 +64,7 @@ template <> struct Num<float> {
     static __device__ __forceinline__ void step(T &x, T &y, T cx, T cy) { chaos::step<float, ARITH_FMA>(x, y, cx, cy); }
     static __device__ __forceinline__ float r2(T x, T y) { return radius2<float, ARITH_FMA>(x, y); }
     static __device__ __forceinline__ bool blockable(T cx, T cy) { return blockable_c(cx, cy); }
+    static __device__ __forceinline__ bool interior(T cx, T cy) { return interior_c(cx, cy); }
 };
 template <> struct Num<double> {
     using T = double;
@@ -72,6 +73,7 @@ template <> struct Num<double> {
     static __device__ __forceinline__ void step(T &x, T &y, T cx, T cy) { chaos::step<double, ARITH_FMA>(x, y, cx, cy); }
     static __device__ __forceinline__ double r2(T x, T y) { return radius2<double, ARITH_FMA>(x, y); }
     static __device__ __forceinline__ bool blockable(T cx, T cy) { return blockable_c(cx, cy); }
+    static __device__ __forceinline__ bool interior(T cx, T cy) { return interior_c(cx, cy); }
 };
 template <> struct Num<FF> {
     using T = FF;
@@ -80,6 +82,7 @@ template <> struct Num<FF> {
     static __device__ __forceinline__ void step(T &x, T &y, T cx, T cy) { ff_step(x, y, cx, cy); }
     static __device__ __forceinline__ float r2(T x, T y) { return ff_radius2(x, y); }
     static __device__ __forceinline__ bool blockable(T cx, T cy) { return blockable_c(cx.hi, cy.hi); }
+    static __device__ __forceinline__ bool interior(T cx, T cy) { return interior_c(cx.hi, cy.hi); }
 };
 
 // Binary64 with the reference's rounding (tier CHAOS_TIER_F64_ROUNDED): the
@@ -96,6 +99,7 @@ template <> struct Num<R64> {
     }
     static __device__ __forceinline__ double r2(T x, T y) { return radius2<double, ARITH_PARITY>(x, y); }
     static __device__ __forceinline__ bool blockable(T cx, T cy) { return blockable_c(cx, cy); }
+    static __device__ __forceinline__ bool interior(T cx, T cy) { return interior_c(cx, cy); }
 };
 template <class N> constexpr bool is_binary64() { return std::is_same<N, double>::value || std::is_same<N, R64>::value; }
 
@@ -206,6 +210,11 @@ template <class N, int K> __global__ void __launch_bounds__(512) k_batch(BatchAr
                         r2 = (float)rr;
                         if (i == max_iter || !(rr < 4.0)) done = true;
                     }
+                }
+                if (!done && P::interior(cx, cy)) {
+                    skipped += max_iter - i;
+                    i = max_iter;
+                    done = true;
                 }
             }
             if (!done && !std::is_same<N, FF>::value) {

@@ -269,8 +269,6 @@ __device__ __forceinline__ void step_contracted4(double &x, double &y, double cx
 // states are compared as bit patterns (on the integer units, beside the
 // binary64 pipe's step), binary32 ones under == (where only a zero's sign
 // can differ between equal values, and it changes no later magnitude).
-constexpr uint32_t CYCLE_SPAN = 16;  // steps between checkpoints in the tested binary32 blocks
-
 __device__ __forceinline__ bool same_state(float a, float b) { return a == b; }
 __device__ __forceinline__ bool same_state(double a, double b)
 {
@@ -312,33 +310,30 @@ template <class T> struct CycleWatch {
 };
 template <class T> constexpr int cycle_blocks() { return sizeof(T) == 8 ? 8 : 1; }
 
-// Up to K steps of the reference loop, each with its own test (binary32
-// frames): stops at a state that tests >= 4 (esc, r2 = its test value) or
-// after `lim` steps when BOUNDED.  Returns the steps taken.  In rounded
-// arithmetic the test's products are the step's own, so a test costs one add,
-// a compare and a branch; a lane that stops waits for its warp at the end of
-// the block.  Exact for every c, with no roll-back or search.
-// With a CycleWatch (unbounded blocks only, K a multiple of CYCLE_SPAN), a
-// checkpoint comes after every CYCLE_SPAN steps; `cyc` reports a repeat.
-template <class R, int A, int K, bool BOUNDED>
-__device__ __forceinline__ uint32_t tested_block(R &x, R &y, R cx, R cy, uint32_t lim, R &r2, bool &esc,
-                                                 CycleWatch<R> *cw = nullptr, bool *cyc = nullptr)
+// Steps with a test after each, from a state that tests below 4 with
+// i < end: until a state tests >= 4 or i reaches `end`.  r2 is the last
+// test's value; (x, y) is the state only where neither happened before a
+// multiple of four steps.  A branch after every step
+// made a step's latency about 76 cycles (a lone warp took 20 us for 500
+// steps); the chain itself is 12, so binary32 steps run in groups of four
+// whose tests only move i, r2 and a flag: the steps past an escape are
+// computed and ignored.  Binary64 tests each step: there a step's pipe time
+// is the longer.
+template <class R, int A>
+__device__ __forceinline__ void tested_steps(R &x, R &y, R cx, R cy, uint32_t &i, uint32_t end, R &r2)
 {
+    constexpr int GROUP = sizeof(R) == 4 ? 4 : 1;
+    bool go = true;
+    do {
 #pragma unroll
-    for (int k = 0; k < K; k++) {
-        if (BOUNDED && (uint32_t)k == lim) return lim;
-        r2 = radius2<R, A>(x, y);
-        if (!(r2 < R(4))) {
-            esc = true;
-            return (uint32_t)k;
+        for (int k = 0; k < GROUP; k++) {
+            step<R, A>(x, y, cx, cy);
+            const R t = radius2<R, A>(x, y);
+            r2 = go ? t : r2;
+            i += go ? 1u : 0u;
+            go = go && t < R(4) && i < end;
         }
-        step<R, A>(x, y, cx, cy);
-        if (!BOUNDED && cw && ((k + 1) % (int)CYCLE_SPAN) == 0 && cw->check(x, y)) {
-            *cyc = true;
-            return (uint32_t)(k + 1);
-        }
-    }
-    return (uint32_t)K;
+    } while (go);
 }
 
 // Escape loop with the reference's semantics:
@@ -353,10 +348,7 @@ __device__ __forceinline__ uint32_t tested_block(R &x, R &y, R cx, R cy, uint32_
 // escape.  Otherwise `blockable` is false and every step is tested.
 // Every kept block ends at a checkpoint of the exact cycle detection
 // (CycleWatch): a state that repeats proves the sample interior.
-// r2_exit is r2 of the final state.  (Tested blocks, which the binary32
-// frame kernel uses, were slower here: a tile's lanes run in lock step, so
-// every lane pays the per-step test for as long as the tile's slowest lane
-// runs, while a roll-back costs only the lane that escaped.)
+// r2_exit is r2 of the final state.
 // Binary64 blocks run step_rounded6 / step_fma3 (the same values as step<>)
 // and are redone with step<> when the integer checks ask for it.  i0 is the
 // iteration count of the state passed in (1 when a Mandelbrot caller starts
@@ -414,12 +406,7 @@ __device__ __forceinline__ uint32_t escape(uint32_t max_iter, R x, R y, R cx, R 
             }
         }
     }
-    while (i < max_iter) {
-        step<R, A>(x, y, cx, cy);
-        ++i;
-        r2 = radius2<R, A>(x, y);
-        if (!(r2 < R(4))) break;
-    }
+    if (i < max_iter) tested_steps<R, A>(x, y, cx, cy, i, max_iter, r2);
     r2_exit = r2;
     return i;
 }
@@ -428,6 +415,40 @@ template <class R> __device__ __forceinline__ bool blockable_c(R cx, R cy)
 {
     return radius2<R, ARITH_PARITY>(cx, cy) <= R(3.99);
 }
+
+// Whether the Mandelbrot orbit of c provably never escapes, in any of the
+// arithmetics here and for any number of iterations: c lies in the main
+// cardioid with the multiplier |mu| of its fixed point at most 1 - 2^-7
+// (c = mu/2 - mu^2/4), or in the period-2 disc with |mu_2| = 4 |c + 1| at
+// most 1 - 2^-6.  There the critical orbit falls into a disc around the
+// attracting cycle that a step maps into itself with room for a step's
+// rounding (at most 2^-21 in binary32), and the rounding errors on the way
+// there add up to less than 2^-12; tests/test_interior_bound.py proves both
+// in ball arithmetic.  The reference's loop then runs to maxIterations, so
+// the answer is known without a step.  Evaluated in binary32 for every type:
+// with s = sqrt(1 - 4c), mu = 1 - s, and |1 - s|^2 <= rho^2 reads
+// 2 Re s - |s|^2 >= 1 - rho^2; the computed side is off by less than 6e-5
+// where the test can pass (Re s >= 2^-7) and the bounds leave 2e-4.
+// Without it a binary32 sample ran until a state repeated bit for bit: on
+// the 1024x1024 frame of the whole set 44.8 of the 49.8 M steps run.
+__device__ __forceinline__ float sqrt_near(float v)  // relative error at most 2^-23
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ bool interior_c(float cx, float cy)
+{
+    constexpr float CARDIOID = 0.0158f;  // > 1 - (1 - 2^-7)^2 = 0.01556
+    constexpr float DISC = 0.0605f;      // < ((1 - 2^-6) / 4)^2 = 0.06056
+    const float y2 = cy * cy;
+    const float a = fmaf(-4.f, cx, 1.f), b2 = 16.f * y2;
+    const float A = sqrt_near(fmaf(a, a, b2));            // |s|^2
+    const float re = sqrt_near(fmaf(0.5f, A, 0.5f * a));  // Re s (NaN where a = -A rounds below 0: no)
+    const float u = cx + 1.f;
+    return fmaf(2.f, re, -A) >= CARDIOID || fmaf(u, u, y2) <= DISC;
+}
+__device__ __forceinline__ bool interior_c(double cx, double cy) { return interior_c((float)cx, (float)cy); }
 
 // ---------------------------------------------------------------------------
 // float-float: a value hi + lo of two binary32 numbers (|lo| <= ulp(hi)/2),
@@ -542,6 +563,7 @@ __device__ __forceinline__ uint32_t escape_ff(uint32_t max_iter, FF x, FF y, FF 
 // returns i.  `jc` is julia_c already converted to Real.
 template <class R, int A, int F> __device__ __forceinline__ uint32_t compute_fractal(uint32_t max_iter, R px, R py, R jcx, R jcy)
 {
+    if (F == FRACTAL_MANDELBROT && interior_c(px, py)) return 0;  // i == max_iter
     if constexpr (A == ARITH_FLOATFLOAT) {
         static_assert(sizeof(R) == 8, "float-float escape loops start from binary64 points");
         const FF fx = ff_from_double(px), fy = ff_from_double(py);

@@ -3,15 +3,16 @@
 //   k_main / k_advanced   reference-mode frames (fractalRenderMain/Advanced,
 //                         gen.cu:168-181, 307-368): persistent warps take 8x4
 //                         tiles from a work counter, one tile = one vote group
-//   k_frame               independent samples (pixel centres or jittered):
-//                         persistent warps with per-lane refill, so a lane whose
-//                         sample escaped takes the next one without waiting for
-//                         the slowest lane of its warp; binary32 samples run
-//                         tested blocks (each step with its own test), binary64
-//                         ones untested blocks with an in-warp search of an
-//                         overshot block
+//   k_frame               independent binary64 samples (pixel centres or
+//                         jittered): persistent warps with per-lane refill, so a
+//                         lane whose sample escaped takes the next one without
+//                         waiting for the slowest lane of its warp; untested
+//                         blocks with an in-warp search of an overshot block
+//   k_frame32             independent binary32 samples: short orbits as they
+//                         come, long ones queued and packed into full warps
 //   k_compose             palette compose (gen.cu:455-475), HBM-bound
 //   k_under_sampled       fractalRenderUnderSampled (gen.cu:478-503)
+#include <algorithm>
 #include <cstdio>
 
 #include "chaos_frame.cuh"
@@ -44,9 +45,10 @@ __device__ __forceinline__ void frame_point(const FrameArgs<R> &a, uint32_t w_ma
     cy = O::fma(-dyp, a.ps, a.center_y);
 }
 
-template <class R, int A, int F, int K> __global__ void __launch_bounds__(PERSIST_THREADS) k_frame(FrameArgs<R> a)
+template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_frame(FrameArgs<double> a)
 {
-    static_assert(sizeof(R) == 4 ? K % CYCLE_SPAN == 0 : K == ESCAPE_BLOCK, "cycle checkpoints at block ends");
+    using R = double;
+    constexpr int K = ESCAPE_BLOCK;
     __shared__ uint32_t s_pal[PALETTE_SMEM];
     const uint32_t *pal = a.palette;
     if (a.rgba && a.palette_len <= PALETTE_SMEM) {
@@ -131,9 +133,15 @@ template <class R, int A, int F, int K> __global__ void __launch_bounds__(PERSIS
                 window = 0;
                 cw.reset(x, y);
                 r2 = radius2<R, A>(x, y);
-                if (i == a.max_iter || !(r2 < R(4))) done = true;
+                if (i == a.max_iter || !(r2 < R(4))) {
+                    done = true;
+                } else if (F == FRACTAL_MANDELBROT && interior_c(cx, cy)) {
+                    skipped += a.max_iter - i;
+                    i = a.max_iter;
+                    done = true;
+                }
             }
-            if (!done && sizeof(R) == 8) {
+            if (!done) {
                 if (!blk) {
                     lim = 1;
                 } else if (window) {
@@ -150,7 +158,7 @@ template <class R, int A, int F, int K> __global__ void __launch_bounds__(PERSIS
         // halves its search window each round without holding up the others.
         const bool stepping = active && !done;
         const bool partial = stepping && lim < (uint32_t)K;
-        const bool any_partial = sizeof(R) == 8 && __any_sync(FULL, partial);
+        const bool any_partial = __any_sync(FULL, partial);
         // K steps of `stepper`, keeping the state after lim steps on partial lanes
         auto run_block = [&](auto stepper) {
             if (any_partial) {
@@ -172,26 +180,10 @@ template <class R, int A, int F, int K> __global__ void __launch_bounds__(PERSIS
                 for (int k = 0; k < K; k++) stepper(x, y);
             }
         };
-        if constexpr (sizeof(R) == 4) {
-            // binary32: tested steps (see tested_block)
-            if (stepping) {
-                const uint32_t rest = a.max_iter - i;
-                bool esc = false, cyc = false;
-                const uint32_t n = rest >= (uint32_t)K
-                                       ? tested_block<R, A, K, false>(x, y, cx, cy, K, r2, esc, &cw, &cyc)
-                                       : tested_block<R, A, K, true>(x, y, cx, cy, rest, r2, esc);
-                i += n;
-                if (cyc) {  // a repeated state: interior
-                    skipped += a.max_iter - i;
-                    i = a.max_iter;
-                }
-                if (esc || i == a.max_iter) done = true;
-            }
-        } else if (stepping) {
+        if (stepping) {
             const R sx = x, sy = y;
-            if constexpr (A == ARITH_PARITY && sizeof(R) == 8) {
-                // binary64: one binary64 operation fewer per step for two integer ones
-                // (binary32 keeps the literal step: there the integer pipe is the busier one)
+            if constexpr (A == ARITH_PARITY) {
+                // one binary64 operation fewer per step for two integer ones
                 uint32_t emin = 0xffffffffu;
                 run_block([&](R &u, R &v) { step_rounded6<R>(u, v, cx, cy, emin); });
                 if (emin < exponent_bits_two<R>()) {
@@ -200,7 +192,7 @@ template <class R, int A, int F, int K> __global__ void __launch_bounds__(PERSIS
                     y = sy;
                     run_block([&](R &u, R &v) { step<R, A>(u, v, cx, cy); });
                 }
-            } else if constexpr (sizeof(R) == 8) {
+            } else {
                 uint32_t emin = 0xffffffffu;
                 run_block([&](R &u, R &v) { step_fma3(u, v, cx, cy, emin); });
                 if (emin == 0u) {
@@ -209,8 +201,6 @@ template <class R, int A, int F, int K> __global__ void __launch_bounds__(PERSIS
                     y = sy;
                     run_block([&](R &u, R &v) { step<R, A>(u, v, cx, cy); });
                 }
-            } else {
-                run_block([&](R &u, R &v) { step<R, A>(u, v, cx, cy); });
             }
             r2 = radius2<R, A>(x, y);
             if (r2 < R(4)) {
@@ -265,6 +255,385 @@ template <class R, int A, int F, int K> __global__ void __launch_bounds__(PERSIS
                 begin = true;
             }
         }
+    }
+    if (a.total) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) iters += __shfl_down_sync(FULL, iters, o);
+        if (lane == 0 && iters) atomicAdd(a.total, iters);
+    }
+    if (a.skipped) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) skipped += __shfl_down_sync(FULL, skipped, o);
+        if (lane == 0 && skipped) atomicAdd(a.skipped, skipped);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Binary32 frames: fresh pixels and long orbits apart
+// ---------------------------------------------------------------------------
+//
+// After interior_c most samples of a view end within a few steps, and the few
+// that go on (samples close to the boundary, interiors of the smaller
+// components) go on for hundreds.  Mixed in one warp, each long orbit held its
+// 31 neighbours to a round of 64 steps.  So a warp takes fresh pixels 32 at a
+// time and gives every sample up to FRESH_STEPS steps; samples still running
+// then wait in the warp's queue in shared memory, and when the queue holds a
+// warp's worth they run by themselves in rounds of 64 steps, lanes that end
+// refilled from the queue, until fewer than REQUEUE lanes are left.  When the
+// fresh pixels are gone the block's waiting orbits are packed into as few
+// warps as hold them, again and again as they end: a warp alone would run its
+// few leftovers, often up to maxIterations, with most lanes idle.
+//
+// Fresh pixels: a fixed share first (batch k of warp w is batch k n_warps + w),
+// the rest claimed 32 at a time from the work counter.  One claim per 32
+// pixels from the start made the counter's address the bottleneck of cheap
+// frames (32768 atomics on one word for 1024x1024 pixels).
+//
+// The bound is issue: 1024x1024 pixels of the whole set, maxIter 1000, take
+// 20 us for the fresh part (360 instructions a batch) and 25 us for the long
+// orbits, whose end is the block with the most of them.  Measured there with
+// the memset of the counter: 85 us with per-lane refill in tested 64-step
+// rounds, 81 with interior_c, 72 with queues alone, 55 with untested blocks for
+// the long orbits, 51 with ended samples written several at a time, 46 with
+// packing and the skew (FRESH_STEPS 16: 49; REQUEUE 12: 49).  256x144 pixels,
+// maxIter 500: 20.6 -> 15.
+constexpr int FRESH_STEPS = 32;
+constexpr int LONG_STEPS = 64;
+constexpr uint32_t REQUEUE = 24;
+constexpr int MAX_EPOCH = 16;         // rounds between packings, at most
+constexpr uint32_t FINISH_LANES = 12;  // samples of a warp that end before any of them is written
+constexpr uint32_t QUEUE = 64;  // entries per warp: at most 31 waiting and 32 fresh
+
+template <bool MULTI> constexpr int frame32_threads() { return MULTI ? 256 : 512; }
+
+template <int A, int F, bool MULTI>
+__global__ void __launch_bounds__(frame32_threads<MULTI>()) k_frame32(FrameArgs<float> a, uint32_t fixed_rounds)
+{
+    constexpr int WORDS = MULTI ? 12 : 6, WARPS = frame32_threads<MULTI>() / 32;
+    __shared__ uint32_t s_pal[PALETTE_SMEM];
+    __shared__ uint32_t s_queue[WARPS][WORDS][QUEUE];
+    __shared__ uint32_t s_count[WARPS];
+    const uint32_t *pal = a.palette;
+    if (a.rgba && a.palette_len <= PALETTE_SMEM) {
+        for (uint32_t k = threadIdx.x; k < a.palette_len; k += blockDim.x) s_pal[k] = a.palette[k];
+        pal = s_pal;
+    }
+    __syncthreads();
+
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t w_magic = div_magic(a.w);
+    const uint32_t wib = threadIdx.x >> 5;
+    uint32_t(*q)[QUEUE] = s_queue[wib];
+    uint32_t qn = 0;  // entries waiting
+    const uint32_t n_warps = gridDim.x * (blockDim.x >> 5);
+    // neighbouring batches go to different blocks, and a block's batches are spread
+    // over the columns of frames of any width (the skew)
+    const uint32_t warp = wib * gridDim.x + (blockIdx.x + 37u * wib) % gridDim.x;
+    const uint32_t claim_base = 32u * n_warps * fixed_rounds;
+    uint32_t round = 0;
+    bool more = true;
+
+    uint32_t pix = 0, s = 0, i = 0;
+    float x = 0.f, y = 0.f, cx = 0.f, cy = 0.f, r2 = 0.f;
+    float acc_v = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+    unsigned long long iters = 0, skipped = 0;
+    const unsigned long long t_start = a.budget_ns ? global_ns() : 0ull;
+
+    // start sample s of pixel pix; true when it ends before its first step
+    auto start = [&]() -> bool {
+        float px, py;
+        frame_point(a, w_magic, pix, s, px, py);
+        i = 0;
+        if (F == FRACTAL_MANDELBROT) {
+            cx = px;
+            cy = py;
+            x = y = 0.f;
+            if (a.max_iter > 0) {  // from z = c, as k_frame
+                x = __fadd_rn(cx, 0.f);
+                y = __fadd_rn(cy, 0.f);
+                i = 1;
+            }
+        } else {
+            x = px;
+            y = py;
+            cx = a.jcx;
+            cy = a.jcy;
+        }
+        r2 = radius2<float, A>(x, y);
+        if (i == a.max_iter || !(r2 < 4.f)) return true;
+        if (F == FRACTAL_MANDELBROT && interior_c(cx, cy)) {
+            skipped += a.max_iter - i;
+            i = a.max_iter;
+            return true;
+        }
+        return false;
+    };
+    // write the sample that ended; true when its pixel is complete
+    auto finish = [&]() -> bool {
+        const bool escaped = i < a.max_iter;
+        const float nu = (a.smooth || a.pixels || a.rgba) ? frame_smooth(i, r2, a.max_iter) : 0.f;
+        const size_t sidx = (size_t)pix * a.spp + s;
+        if (a.counts) a.counts[sidx] = i;
+        if (a.smooth) a.smooth[sidx] = nu;
+        iters += i;
+        const float v = escaped ? nu : (F == FRACTAL_MANDELBROT ? 0.f : (float)a.max_iter);
+        acc_v = __fadd_rn(MULTI ? acc_v : 0.f, v);
+        if (a.rgba) {
+            float ch[4];
+            if (escaped) {
+                frame_palette_lerp(pal, a.palette_len, nu, ch);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; k++) ch[k] = (float)((a.interior_rgba >> (8 * k)) & 255u);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) acc[k] = __fadd_rn(MULTI ? acc[k] : 0.f, ch[k]);
+        }
+        if (MULTI && ++s < a.spp) return false;
+        if (a.pixels) {
+            uint32_t px, py;
+            divmod_magic(pix, a.w, w_magic, py, px);
+            store_pixel(pixel_ptr(a.pixels, a.pixels_pitch, px, py),
+                        make_pixel(__fdiv_rn(acc_v, (float)a.spp), (float)a.spp));
+        }
+        if (a.rgba) a.rgba[pix] = frame_pack_rgba(acc, a.spp);
+        return true;
+    };
+    // lanes with `put` append their samples to the queue
+    auto push = [&](bool put) {
+        const uint32_t mask = __ballot_sync(FULL, put);
+        if (put) {
+            const uint32_t at = qn + (uint32_t)__popc(mask & lt_mask);
+            q[0][at] = __float_as_uint(x);
+            q[1][at] = __float_as_uint(y);
+            q[2][at] = __float_as_uint(cx);
+            q[3][at] = __float_as_uint(cy);
+            q[4][at] = i;
+            q[5][at] = pix;
+            if constexpr (MULTI) {
+                q[6][at] = s;
+                q[7][at] = __float_as_uint(acc_v);
+#pragma unroll
+                for (int k = 0; k < 4; k++) q[8 + k][at] = __float_as_uint(acc[k]);
+            }
+        }
+        qn += (uint32_t)__popc(mask);
+        __syncwarp();
+    };
+    auto pop = [&](uint32_t(*q)[QUEUE], uint32_t at) {
+        x = __uint_as_float(q[0][at]);
+        y = __uint_as_float(q[1][at]);
+        cx = __uint_as_float(q[2][at]);
+        cy = __uint_as_float(q[3][at]);
+        i = q[4][at];
+        pix = q[5][at];
+        if constexpr (MULTI) {
+            s = q[6][at];
+            acc_v = __uint_as_float(q[7][at]);
+#pragma unroll
+            for (int k = 0; k < 4; k++) acc[k] = __uint_as_float(q[8 + k][at]);
+        }
+    };
+
+    // a round of a long orbit; true when the sample ended.  While |c| allows,
+    // blocks of 16 untested steps as in escape(), with no branch between them: the
+    // state after the last block that ended below 4 is kept, and a block that
+    // overshot is gone over again with tests, by all the lanes that overshot in
+    // the round together.
+    CycleWatch<float> cw;
+    auto long_round = [&]() -> bool {
+        const uint32_t rest = a.max_iter - i;
+        bool tested = true;
+        if (rest >= (uint32_t)ESCAPE_BLOCK && blockable_c(cx, cy)) {
+            float kx = x, ky = y;
+            uint32_t n = 0;
+            bool ok = true, cyc = false;
+#pragma unroll 1
+            for (uint32_t end = ESCAPE_BLOCK; end <= (uint32_t)LONG_STEPS; end += ESCAPE_BLOCK) {
+#pragma unroll
+                for (int k = 0; k < ESCAPE_BLOCK; k++) step<float, A>(x, y, cx, cy);
+                ok = ok && radius2<float, A>(x, y) < 4.f && end <= rest;
+                cyc = cyc || (ok && same_state(x, cw.sx) && same_state(y, cw.sy));  // a repeated state: interior
+                cw.ck += ok ? 1u : 0u;
+                const bool save = ok && cw.ck == cw.save_at;
+                cw.sx = save ? x : cw.sx;
+                cw.sy = save ? y : cw.sy;
+                cw.save_at <<= save ? 1 : 0;
+                kx = ok ? x : kx;
+                ky = ok ? y : ky;
+                n = ok ? end : n;
+            }
+            x = kx;
+            y = ky;
+            i += n;
+            if (cyc) {
+                skipped += a.max_iter - i;
+                i = a.max_iter;
+            }
+            if (i == a.max_iter) return true;
+            tested = n < (uint32_t)LONG_STEPS && n + (uint32_t)ESCAPE_BLOCK <= rest;
+        }
+        if (tested) {
+            tested_steps<float, A>(x, y, cx, cy, i, min(i + (uint32_t)LONG_STEPS, a.max_iter), r2);
+            if (!(r2 < 4.f) || i == a.max_iter) return true;
+            if (cw.check(x, y)) {
+                skipped += a.max_iter - i;
+                i = a.max_iter;
+                return true;
+            }
+        }
+        return false;
+    };
+    // the samples that ended: written, the pixel's next sample started; true
+    // when the pixel is complete
+    auto finish_ended = [&]() -> bool {
+        do {
+            if (finish()) return true;
+        } while (start());
+        cw.reset(x, y);
+        return false;
+    };
+
+    bool late = false;
+    while (!late) {
+        // ---- fresh pixels
+        while (more && qn < 32u) {
+            // a time limit: the warp stops where it is (its samples in flight stay unwritten)
+            if ((late = out_of_time(a.budget_ns, t_start, a.status, lane))) break;
+            uint32_t base = 0;
+            if (round < fixed_rounds) {
+                base = 32u * (round++ * n_warps + warp);
+            } else {
+                if (lane == 0) base = claim_base + atomicAdd(a.counter, 32u);
+                base = __shfl_sync(FULL, base, 0);
+            }
+            if (base >= a.n_pix) {
+                more = false;
+                break;
+            }
+            pix = base + lane;
+            bool live = pix < a.n_pix, running = false, put = false;
+            s = 0;
+            acc_v = 0.f;
+            acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+            do {
+                if (live) {
+                    bool ended = start();
+                    if (!ended) {
+                        const uint32_t end = min(i + (uint32_t)FRESH_STEPS, a.max_iter);
+                        tested_steps<float, A>(x, y, cx, cy, i, end, r2);
+                        ended = !(r2 < 4.f) || i == a.max_iter;
+                    }
+                    if (ended) {
+                        live = !finish();
+                    } else {
+                        put = true;
+                        live = false;
+                    }
+                }
+                running = MULTI && __any_sync(FULL, live);
+            } while (running);
+            push(put);
+        }
+        if (late || !more) break;
+        // ---- long orbits: a warp's worth of them
+        qn -= 32u;
+        pop(q, qn + lane);
+        __syncwarp();
+        bool on = true, ended = false;
+        cw.reset(x, y);
+        for (;;) {
+            if ((late = out_of_time(a.budget_ns, t_start, a.status, lane))) break;
+            if (on && !ended) ended = long_round();
+            const uint32_t end_mask = __ballot_sync(FULL, ended);
+            const uint32_t running = (uint32_t)__popc(__ballot_sync(FULL, on && !ended));
+            if ((uint32_t)__popc(end_mask) < FINISH_LANES && running >= REQUEUE) continue;
+            if (ended) {
+                on = !finish_ended();
+                ended = false;
+            }
+            const uint32_t free_mask = __ballot_sync(FULL, !on);
+            if (free_mask && qn) {
+                const uint32_t k = (uint32_t)__popc(free_mask & lt_mask);
+                const uint32_t take = min((uint32_t)__popc(free_mask), qn);
+                if (!on && k < take) {
+                    pop(q, qn - 1u - k);
+                    cw.reset(x, y);
+                    on = true;
+                }
+                qn -= take;
+                __syncwarp();
+            }
+            if ((uint32_t)__popc(__ballot_sync(FULL, on)) < REQUEUE) {
+                push(on);
+                break;
+            }
+        }
+    }
+    // ---- the block's remaining orbits, one per thread (at most 31 a warp), packed
+    // into as few warps as hold them every `epoch` rounds
+    if (lane == 0) s_count[wib] = late ? 0u : qn;
+    __syncthreads();
+    uint32_t left = 0;
+#pragma unroll
+    for (int k = 0; k < WARPS; k++) left += s_count[k];
+    bool on = threadIdx.x < left, ended = false;
+    if (on) {
+        uint32_t w = 0, at = threadIdx.x;
+        while (at >= s_count[w]) at -= s_count[w++];
+        pop(s_queue[w], at);
+        cw.reset(x, y);
+    }
+    int epoch = 2;
+    while (left) {
+        late = out_of_time(a.budget_ns, t_start, a.status, lane);
+        for (int k = 0; k < epoch && __any_sync(FULL, on && !ended); k++)
+            if (on && !ended) ended = long_round();
+        epoch = min(2 * epoch, MAX_EPOCH);  // orbits end at a falling rate
+        if (ended) {
+            on = !finish_ended();
+            ended = false;
+        }
+        const uint32_t mask = __ballot_sync(FULL, on && !late);
+        __syncthreads();  // the last epoch's queue and counts have been read
+        if (lane == 0) s_count[wib] = (uint32_t)__popc(mask);
+        __syncthreads();
+        uint32_t at = (uint32_t)__popc(mask & lt_mask), now = 0;
+#pragma unroll
+        for (int k = 0; k < WARPS; k++) {
+            at += (uint32_t)k < wib ? s_count[k] : 0u;
+            now += s_count[k];
+        }
+        const bool pack = (now + 31u) / 32u < (left + 31u) / 32u;
+        left = now;
+        if (!pack) {
+            on = on && !late;
+            continue;
+        }
+        // words 0.. of every waiting orbit at [word][at], then its cycle watch
+        uint32_t *flat = &s_queue[0][0][0];
+        constexpr uint32_t T = frame32_threads<MULTI>();
+        static_assert((WORDS + 4) * T <= WARPS * WORDS * QUEUE, "a packed orbit per thread fits the queues");
+        auto swap_words = [&](bool put, uint32_t e) {
+            auto word = [&](uint32_t k, auto &v) {
+                if (put)
+                    memcpy(&flat[k * T + e], &v, 4);
+                else
+                    memcpy(&v, &flat[k * T + e], 4);
+            };
+            word(0, x), word(1, y), word(2, cx), word(3, cy), word(4, i), word(5, pix);
+            if constexpr (MULTI) {
+                word(6, s), word(7, acc_v);
+#pragma unroll
+                for (int k = 0; k < 4; k++) word(8 + k, acc[k]);
+            }
+            word(WORDS, cw.sx), word(WORDS + 1, cw.sy), word(WORDS + 2, cw.ck), word(WORDS + 3, cw.save_at);
+        };
+        if ((mask >> lane) & 1u) swap_words(true, at);
+        __syncthreads();
+        on = threadIdx.x < left;
+        if (on) swap_words(false, threadIdx.x);
     }
     if (a.total) {
 #pragma unroll
@@ -373,29 +742,49 @@ cudaError_t launch_advanced(const AdvancedArgs<R> &a, int arith, int fractal, in
                                     : launch_advanced_t<R, ARITH_FMA, FRACTAL_MANDELBROT>(a, sms, s);
 }
 
-// Block length per arithmetic width: binary32 frames run tested blocks of 64
-// steps (on the 1024x1024 frame with a mean escape of 173 iterations, 16, 32,
-// 64 and 128 steps gave 1499, 1669, 1746 and 1620 Gpixel-iter/s); binary64
-// runs untested blocks of 16.
-template <class R> constexpr int frame_block() { return sizeof(R) == 4 ? 64 : ESCAPE_BLOCK; }
-
-template <class R, int A, int F> static cudaError_t launch_frame_t(const FrameArgs<R> &a, int sms, cudaStream_t s)
+template <int A, int F> static cudaError_t launch_frame64(const FrameArgs<double> &a, int sms, cudaStream_t s)
 {
-    constexpr int K = frame_block<R>();
-    static const int occ = occupancy(k_frame<R, A, F, K>, PERSIST_THREADS);
+    static const int occ = occupancy(k_frame<A, F>, PERSIST_THREADS);
     unsigned long long warps = ((unsigned long long)a.n_pix + 31ull) / 32ull;
-    k_frame<R, A, F, K><<<grid_for(warps, occ, sms), PERSIST_THREADS, 0, s>>>(a);
+    k_frame<A, F><<<grid_for(warps, occ, sms), PERSIST_THREADS, 0, s>>>(a);
     return cudaGetLastError();
+}
+
+template <int A, int F, bool MULTI> static cudaError_t launch_frame32_t(const FrameArgs<float> &a, int sms, cudaStream_t s)
+{
+    constexpr int threads = frame32_threads<MULTI>();
+    static const int occ = occupancy(k_frame32<A, F, MULTI>, threads);
+    const unsigned long long batches = ((unsigned long long)a.n_pix + 31ull) / 32ull, warps = threads / 32;
+    const unsigned long long fill = (unsigned long long)occ * (unsigned long long)sms;
+    const unsigned grid = (unsigned)std::min(fill, batches);
+    const unsigned long long n_warps = (unsigned long long)grid * warps;
+    uint32_t fixed = (uint32_t)(batches * 5ull / 8ull / n_warps);  // rounds of fixed batches
+    if (fixed < 1) fixed = 1;
+    k_frame32<A, F, MULTI><<<grid, threads, 0, s>>>(a, fixed);
+    return cudaGetLastError();
+}
+template <int A, int F> static cudaError_t launch_frame32(const FrameArgs<float> &a, int sms, cudaStream_t s)
+{
+    return a.spp > 1 ? launch_frame32_t<A, F, true>(a, sms, s) : launch_frame32_t<A, F, false>(a, sms, s);
 }
 
 template <class R>
 cudaError_t launch_frame(const FrameArgs<R> &a, int arith, int fractal, int sms, cudaStream_t s)
 {
-    if (arith == ARITH_PARITY)
-        return fractal == FRACTAL_JULIA ? launch_frame_t<R, ARITH_PARITY, FRACTAL_JULIA>(a, sms, s)
-                                        : launch_frame_t<R, ARITH_PARITY, FRACTAL_MANDELBROT>(a, sms, s);
-    return fractal == FRACTAL_JULIA ? launch_frame_t<R, ARITH_FMA, FRACTAL_JULIA>(a, sms, s)
-                                    : launch_frame_t<R, ARITH_FMA, FRACTAL_MANDELBROT>(a, sms, s);
+    const bool julia = fractal == FRACTAL_JULIA;
+    if constexpr (sizeof(R) == 4) {
+        if (arith == ARITH_PARITY)
+            return julia ? launch_frame32<ARITH_PARITY, FRACTAL_JULIA>(a, sms, s)
+                         : launch_frame32<ARITH_PARITY, FRACTAL_MANDELBROT>(a, sms, s);
+        return julia ? launch_frame32<ARITH_FMA, FRACTAL_JULIA>(a, sms, s)
+                     : launch_frame32<ARITH_FMA, FRACTAL_MANDELBROT>(a, sms, s);
+    } else {
+        if (arith == ARITH_PARITY)
+            return julia ? launch_frame64<ARITH_PARITY, FRACTAL_JULIA>(a, sms, s)
+                         : launch_frame64<ARITH_PARITY, FRACTAL_MANDELBROT>(a, sms, s);
+        return julia ? launch_frame64<ARITH_FMA, FRACTAL_JULIA>(a, sms, s)
+                     : launch_frame64<ARITH_FMA, FRACTAL_MANDELBROT>(a, sms, s);
+    }
 }
 
 cudaError_t launch_compose(const ComposeArgs &a, cudaStream_t s)

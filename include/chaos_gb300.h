@@ -275,7 +275,8 @@ typedef struct chaos_frame_out {
     unsigned long long *rebases; /* perturbation tiers: glitch repairs (rebasing events) */
     /* one uint64 the kernel adds the iterations it did not run to: a sample
      * whose state repeats bit for bit is interior (the iteration is
-     * deterministic), so it counts max_iterations without running the rest
+     * deterministic), or a point inside the main cardioid or the period-2
+     * disc, so it counts max_iterations without running the rest
      * (binary32 and binary64 tiers; total_iterations counts it in full) */
     unsigned long long *cycle_skipped;
     /* one uint32 the kernel ORs CHAOS_STATUS_* bits into (zeroed by the
@@ -381,8 +382,9 @@ int chaos_batch_tiers(const chaos_batch *batch, uint32_t *tiers, uint32_t n);
 int chaos_batch_total(const chaos_batch *batch, unsigned long long **device_total);
 /* The same total copied to host memory (synchronises the device). */
 int chaos_batch_read_total(const chaos_batch *batch, unsigned long long *total);
-/* Iterations of the last launch not run because a sample's state repeated
- * bit for bit (interior; counted in full in the total), copied to the host. */
+/* Iterations of the last launch not run because a sample was proven interior
+ * (a state that repeated bit for bit, a point inside the main cardioid or the
+ * period-2 disc; counted in full in the total), copied to the host. */
 int chaos_batch_read_cycle_skipped(const chaos_batch *batch, unsigned long long *skipped);
 /* CHAOS_STATUS_* bits of the last launch (after it has finished): 0, or
  * CHAOS_STATUS_TIMEOUT when config->time_limit_s ran out. */
