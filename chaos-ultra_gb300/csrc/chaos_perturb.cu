@@ -46,7 +46,6 @@
 #include <cstring>
 #include <mutex>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/chaos_gb300.h"
@@ -729,92 +728,139 @@ int api_orbit_create_d(double center_x, double center_y, uint32_t bits, uint32_t
 }
 }  // namespace chaos
 
-// A composed block: L linear steps w <- a_j w + u (a_j = 2Z_j) from m as
-// w <- P w + Q u.
-struct BlockMap {
-    double px = 0, py = 0, qx = 0, qy = 0;
+namespace chaos {
+
+// The tables of an orbit that follow from its binary64 values, one thread per
+// index m and difference type (blockIdx.y: 0 binary32, 1 binary64).
+struct OrbitTables {
+    const double2 *z64;
+    uint32_t n;
+    float2 *z32, *z2;
+    double2 *z2_64;
+    float4 *bla16, *bla64;
+    char2 *lin_lim;
+    double2 *bla16d, *bla64d;
+    char2 *lin_limd;
 };
 
-// The 16- and 64-step blocks from every index m, composed in binary64 from
-// a2[j] = 2Z_j as the kernel holds it, and where each may stand in for full
-// steps (lim[m] = (l16, l64)).  With w_j = P_(m->j) w + Q_(m->j) u the
-// difference at step j and M = max(|w|, |u|) componentwise,
+// The 16- and 64-step blocks from every index m: L linear steps w <- a_j w + u
+// (a_j = 2Z_j as the kernel of the type holds it) composed in binary64 as
+// w <- P w + Q u, and where each may stand in for full steps
+// (lim[m] = (l16, l64)).  With w_j = P_(m->j) w + Q_(m->j) u the difference
+// at step j and M = max(|w|, |u|) componentwise,
 //     |2^e w_j| < 2^(e + ilogb(M) + 1.5) (|P_j| + |Q_j|)
 //              <= 2^(e + ilogb(M) + 1.5) sqrt(2 (|P_j|^2 + |Q_j|^2)),
 // and the quadratic term of step j is below the arithmetic's rounding (2^-p
 // relative) when that stays below 2^-p |Z_j| (p = slack - 1.5): for
 // j = m..m+L that holds when
 //     e + ilogb(M) <= floor(log2(rho) / 2 - slack),
-//     rho = min_j |Z_j|^2 / (2 (|P_j|^2 + |Q_j|^2))   (zz[j] = |Z_j|^2).
-// No test may fire inside: ev[j] is false for j = m+1..m+L (the caller sets
-// it where |Z_j|^2 >= 3.99 or < 2^-98, margins on the escape and glitch tests,
-// which then see z_j = Z_j to the arithmetic's precision), the block ends
-// before the orbit's last index, and Z_m != 0.  A 64-step block also keeps
-// |w| below 2^127 at its end (|w|, |u| <= 2^25 before it):
-// 2 (|P|^2 + |Q|^2) <= 2^200.  A bound below -127 is stored as none.
-static void compose_blocks(const std::vector<double2> &a2, const std::vector<double> &zz,
-                           const std::vector<char> &ev, double slack, std::vector<BlockMap> &b16,
-                           std::vector<BlockMap> &b64, std::vector<char2> &lim)
+//     rho = min_j |Z_j|^2 / (2 (|P_j|^2 + |Q_j|^2))   (zz = |Z_j|^2).
+// No test may fire inside: no event at j = m+1..m+L (|Z_j|^2 >= 3.99 or
+// < 2^-98, margins on the escape and glitch tests, which then see z_j = Z_j to
+// the arithmetic's precision), the block ends before the orbit's last index,
+// and Z_m != 0.  A 64-step block also keeps |w| below 2^127 at its end
+// (|w|, |u| <= 2^25 before it): 2 (|P|^2 + |Q|^2) <= 2^200.  A bound below -127
+// is stored as none.
+//
+// Bound: the binary64 pipe's latency, 15 operations a step for 64 steps
+// (about 35 us for orbits that fill less than the chip, whatever their
+// length; the least ratio is found by cross-multiplication, its one division
+// at the end).  On the host, 931 indices took 0.2 to 0.4 ms on up to eight
+// threads for each type, and 156 bytes an index went to the device instead of
+// 24.  Blocks of 64 threads: an orbit of 1000 entries spreads over 32 SMs.
+constexpr int TABLE_THREADS = 64, TABLE_SPAN = TABLE_THREADS + 65;
+__global__ void __launch_bounds__(TABLE_THREADS) k_orbit_tables(OrbitTables t)
 {
-    const size_t n = a2.size(), last = n - 1;
-    b16.assign(n, BlockMap());
-    b64.assign(n, BlockMap());
-    lim.assign(n, make_char2((signed char)LIN_NONE, (signed char)LIN_NONE));
-    auto lim_of = [slack](double rho) {
-        if (!(rho > 0.0) || !std::isfinite(rho)) return (int)LIN_NONE;
-        const double l = std::floor(0.5 * std::log2(rho) - slack);
-        return l < -127.0 ? (int)LIN_NONE : (int)std::min(127.0, l);
-    };
-    auto part = [&](size_t m0, size_t m1) {
-        for (size_t m = m0; m < m1; m++) {
-            double px = 1.0, py = 0.0, qx = 0.0, qy = 0.0;
-            bool ok16 = m + 16 < last && zz[m] > 0.0, ok64 = m + 64 < last && zz[m] > 0.0;
-            double rho = INFINITY, rho16 = INFINITY;
-            for (size_t j = m; j <= m + 64 && j < n; j++) {
-                if (j > m && ev[j]) {
-                    if (j <= m + 16) ok16 = false;
-                    ok64 = false;
-                }
-                if (!ok64 && j > m + 16) break;
-                rho = std::min(rho, zz[j] / (2.0 * (px * px + py * py + qx * qx + qy * qy)));
-                if (j == m + 16) {
-                    rho16 = rho;
-                    b16[m] = BlockMap{px, py, qx, qy};
-                    if (!ok64) break;
-                }
-                if (j == m + 64) {
-                    if (!(2.0 * (px * px + py * py + qx * qx + qy * qy) <= 0x1p200)) ok64 = false;
-                    b64[m] = BlockMap{px, py, qx, qy};
-                    break;
-                }
-                const double ax = a2[j].x, ay = a2[j].y;
-                const double npx = ax * px - ay * py, npy = ax * py + ay * px;
-                const double nqx = ax * qx - ay * qy + 1.0, nqy = ax * qy + ay * qx;
-                px = npx;
-                py = npy;
-                qx = nqx;
-                qy = nqy;
+    __shared__ double2 s_a[TABLE_SPAN];
+    __shared__ double s_zz[TABLE_SPAN];
+    __shared__ uint8_t s_ev[TABLE_SPAN];
+    const bool wide = blockIdx.y != 0;
+    const uint32_t m0 = blockIdx.x * TABLE_THREADS, last = t.n - 1u;
+    for (uint32_t k = threadIdx.x; k < (uint32_t)TABLE_SPAN && m0 + k < t.n; k += TABLE_THREADS) {
+        const double2 z = t.z64[m0 + k];
+        double zx = z.x, zy = z.y;
+        bool ev;
+        if (wide) {
+            const double r2 = __fma_rn(zx, zx, __dmul_rn(zy, zy));
+            ev = !(r2 < 3.99) || r2 < 0x1p-98;
+        } else {
+            const float fx = (float)zx, fy = (float)zy;
+            const float r2 = __fmaf_rn(fx, fx, __fmul_rn(fy, fy));
+            ev = !(r2 < 3.99f) || r2 < 0x1p-98f;
+            zx = fx;
+            zy = fy;
+            if (k < (uint32_t)TABLE_THREADS) {
+                t.z32[m0 + k] = make_float2(fx, fy);
+                t.z2[m0 + k] = make_float2(2.f * fx, 2.f * fy);
             }
-            lim[m] = make_char2((signed char)(ok16 ? lim_of(rho16) : LIN_NONE), (signed char)(ok64 ? lim_of(rho) : LIN_NONE));
         }
-    };
-    // the indices are independent: they are split over up to 8 host threads
-    // (one per 256 indices); a thread that cannot start leaves its share here
-    const size_t count = n >= 16 ? n - 15 : 0;
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const size_t parts = std::min<size_t>(std::min(8u, hw), std::max<size_t>(1, count / 256));
-    std::vector<std::thread> pool;
-    for (size_t t = 1; t < parts; t++) {
-        const size_t m0 = count * t / parts, m1 = count * (t + 1) / parts;
-        try {
-            pool.emplace_back(part, m0, m1);
-        } catch (...) {
-            part(m0, m1);
-        }
+        s_a[k] = make_double2(2.0 * zx, 2.0 * zy);
+        s_zz[k] = __fma_rn(zx, zx, __dmul_rn(zy, zy));
+        s_ev[k] = ev;
+        if (wide && k < (uint32_t)TABLE_THREADS) t.z2_64[m0 + k] = s_a[k];
     }
-    part(0, count / parts);
-    for (std::thread &th : pool) th.join();
+    __syncthreads();
+    const uint32_t m = m0 + threadIdx.x;
+    if (m >= t.n) return;
+    const double2 *a = s_a + threadIdx.x;
+    const double *zz = s_zz + threadIdx.x;
+    const uint8_t *ev = s_ev + threadIdx.x;
+    double px = 1.0, py = 0.0, qx = 0.0, qy = 0.0;
+    double b16[4] = {0.0, 0.0, 0.0, 0.0}, b64[4] = {0.0, 0.0, 0.0, 0.0};
+    bool ok16 = m + 16u < last && zz[0] > 0.0, ok64 = m + 64u < last && zz[0] > 0.0;
+    double num = INFINITY, den = 1.0, rho16 = 0.0;  // the least ratio so far, num / den
+    const uint32_t steps = min(64u, last - m);
+    for (uint32_t k = 0; k <= steps; k++) {
+        if (k > 0 && ev[k]) {
+            if (k <= 16u) ok16 = false;
+            ok64 = false;
+        }
+        if (!ok64 && k > 16u) break;
+        const double norm =
+            2.0 * __fma_rn(qy, qy, __fma_rn(qx, qx, __fma_rn(px, px, __dmul_rn(py, py))));
+        if (__dmul_rn(zz[k], den) < __dmul_rn(num, norm)) {
+            num = zz[k];
+            den = norm;
+        }
+        if (k == 16u) {
+            rho16 = num / den;
+            b16[0] = px, b16[1] = py, b16[2] = qx, b16[3] = qy;
+            if (!ok64) break;
+        }
+        if (k == 64u) {
+            if (!(norm <= 0x1p200)) ok64 = false;
+            b64[0] = px, b64[1] = py, b64[2] = qx, b64[3] = qy;
+            break;
+        }
+        const double ax = a[k].x, ay = a[k].y;
+        const double npx = __fma_rn(ax, px, -__dmul_rn(ay, py)), npy = __fma_rn(ax, py, __dmul_rn(ay, px));
+        const double nqx = __dadd_rn(__fma_rn(ax, qx, -__dmul_rn(ay, qy)), 1.0);
+        const double nqy = __fma_rn(ax, qy, __dmul_rn(ay, qx));
+        px = npx;
+        py = npy;
+        qx = nqx;
+        qy = nqy;
+    }
+    auto lim_of = [&](bool ok, double rho) -> signed char {
+        if (!ok || !(rho > 0.0) || isinf(rho)) return (signed char)LIN_NONE;
+        const double l = floor(0.5 * log2(rho) - (wide ? 54.5 : 25.5));
+        return (signed char)(l < -127.0 ? (double)LIN_NONE : fmin(127.0, l));
+    };
+    const char2 lim = make_char2(lim_of(ok16, rho16), lim_of(ok64, ok64 ? num / den : 0.0));
+    if (wide) {
+        t.bla16d[2u * m] = make_double2(b16[0], b16[1]);
+        t.bla16d[2u * m + 1u] = make_double2(b16[2], b16[3]);
+        t.bla64d[2u * m] = make_double2(b64[0], b64[1]);
+        t.bla64d[2u * m + 1u] = make_double2(b64[2], b64[3]);
+        t.lin_limd[m] = lim;
+    } else {
+        t.bla16[m] = make_float4((float)b16[0], (float)b16[1], (float)b16[2], (float)b16[3]);
+        t.bla64[m] = make_float4((float)b64[0], (float)b64[1], (float)b64[2], (float)b64[3]);
+        t.lin_lim[m] = lim;
+    }
 }
+
+}  // namespace chaos
 
 static int orbit_compute(const BigFix &cx, const BigFix &cy, int limbs, uint32_t max_iterations, chaos_orbit **out)
 {
@@ -841,81 +887,26 @@ static int orbit_compute(const BigFix &cx, const BigFix &cy, int limbs, uint32_t
             break;
         }
     }
-    std::vector<float2> z32(z64.size()), z2(z64.size());
-    for (size_t k = 0; k < z64.size(); k++) {
-        z32[k] = make_float2((float)z64[k].x, (float)z64[k].y);
-        z2[k] = make_float2(2.f * z32[k].x, 2.f * z32[k].y);
-    }
-    // the composed 16- and 64-step blocks of binary32 differences, from 2Z_j
-    // as that kernel holds it (binary32) and its |Z_j|^2 and tests
-    std::vector<float4> bla16(z64.size(), make_float4(0.f, 0.f, 0.f, 0.f));
-    std::vector<float4> bla64(z64.size(), make_float4(0.f, 0.f, 0.f, 0.f));
-    std::vector<char2> lin_lim;
-    {
-        std::vector<double2> a2(z64.size());
-        std::vector<double> zz(z64.size());
-        std::vector<char> ev(z64.size());
-        for (size_t j = 0; j < z64.size(); j++) {
-            a2[j] = make_double2(z2[j].x, z2[j].y);
-            zz[j] = (double)z32[j].x * z32[j].x + (double)z32[j].y * z32[j].y;
-            const float r2 = std::fmaf(z32[j].x, z32[j].x, z32[j].y * z32[j].y);
-            ev[j] = !(r2 < 3.99f) || r2 < 0x1p-98f;
-        }
-        std::vector<BlockMap> b16, b64;
-        compose_blocks(a2, zz, ev, 25.5, b16, b64, lin_lim);
-        for (size_t m = 0; m < z64.size(); m++) {
-            bla16[m] = make_float4((float)b16[m].px, (float)b16[m].py, (float)b16[m].qx, (float)b16[m].qy);
-            bla64[m] = make_float4((float)b64[m].px, (float)b64[m].py, (float)b64[m].qx, (float)b64[m].qy);
-        }
-    }
     // next_event[m]: first index j >= m where a rescaled step's test can fire,
-    // evaluated as the kernel does (binary32 |Z_j|^2 with one fused add)
-    std::vector<uint32_t> next_event(z64.size());
-    {
-        const size_t last = z64.size() - 1;
-        uint32_t next = (uint32_t)last;
-        for (size_t j = last + 1; j-- > 0;) {
-            const float r2 = std::fmaf(z32[j].x, z32[j].x, z32[j].y * z32[j].y);
-            if (j == last || !(r2 < 4.f) || r2 < 0x1p-100f) next = (uint32_t)j;
-            next_event[j] = next;
-        }
-    }
+    // evaluated as the kernel does (binary32 |Z_j|^2 with one fused add).
     // next_event64[m]: first index j >= m where a binary64 linear step from or to
     // j may differ from the full step: the orbit's end, |Z|^2 >= 4 (as the
     // kernel's escape test computes it), or a component of Z below 2^-20
-    std::vector<double2> z2_64(z64.size());
-    std::vector<uint32_t> next_event64(z64.size());
+    const size_t count = z64.size();
+    std::vector<uint32_t> next_event(count), next_event64(count);
     {
-        const size_t last = z64.size() - 1;
-        uint32_t next = (uint32_t)last;
-        for (size_t j = last + 1; j-- > 0;) {
+        const size_t last = count - 1;
+        uint32_t next = (uint32_t)last, next64 = (uint32_t)last;
+        for (size_t j = count; j-- > 0;) {
             const double zx = z64[j].x, zy = z64[j].y;
-            z2_64[j] = make_double2(2.0 * zx, 2.0 * zy);
-            const double r2 = std::fma(zx, zx, zy * zy);
-            if (j == last || !(r2 < 4.0) || !(std::fabs(zx) >= 0x1p-20) || !(std::fabs(zy) >= 0x1p-20))
-                next = (uint32_t)j;
-            next_event64[j] = next;
-        }
-    }
-    // the same blocks for binary64 differences, from the binary64 orbit, with
-    // binary64 rounding (2^-53 in place of 2^-24)
-    std::vector<double2> bla16d(2 * z64.size()), bla64d(2 * z64.size());
-    std::vector<char2> lin_limd;
-    {
-        std::vector<double> zz(z64.size());
-        std::vector<char> ev(z64.size());
-        for (size_t j = 0; j < z64.size(); j++) {
-            zz[j] = z64[j].x * z64[j].x + z64[j].y * z64[j].y;
-            const double r2 = std::fma(z64[j].x, z64[j].x, z64[j].y * z64[j].y);
-            ev[j] = !(r2 < 3.99) || r2 < 0x1p-98;
-        }
-        std::vector<BlockMap> b16, b64;
-        compose_blocks(z2_64, zz, ev, 54.5, b16, b64, lin_limd);
-        for (size_t m = 0; m < z64.size(); m++) {
-            bla16d[2 * m] = make_double2(b16[m].px, b16[m].py);
-            bla16d[2 * m + 1] = make_double2(b16[m].qx, b16[m].qy);
-            bla64d[2 * m] = make_double2(b64[m].px, b64[m].py);
-            bla64d[2 * m + 1] = make_double2(b64[m].qx, b64[m].qy);
+            const float fx = (float)zx, fy = (float)zy;
+            const float r2 = std::fmaf(fx, fx, fy * fy);
+            if (j == last || !(r2 < 4.f) || r2 < 0x1p-100f) next = (uint32_t)j;
+            const double r2d = std::fma(zx, zx, zy * zy);
+            if (j == last || !(r2d < 4.0) || !(std::fabs(zx) >= 0x1p-20) || !(std::fabs(zy) >= 0x1p-20))
+                next64 = (uint32_t)j;
+            next_event[j] = next;
+            next_event64[j] = next64;
         }
     }
 
@@ -928,41 +919,51 @@ static int orbit_compute(const BigFix &cx, const BigFix &cy, int limbs, uint32_t
     o->bits = (uint32_t)(64 * limbs);
     o->center_x = bigfix_to_double(cx);
     o->center_y = bigfix_to_double(cy);
-    // every table in one device allocation, filled by one copy from one host
-    // image (256-byte aligned parts): an orbit is made per zoom step or batch
-    std::vector<unsigned char> image;
-    image.reserve(z64.size() * 160 + 12 * 256);
-    auto stage = [&image](const auto &v) -> size_t {
-        const size_t at = image.size(), bytes = v.size() * sizeof(v[0]);
-        image.resize((at + bytes + 255) & ~(size_t)255);
-        if (bytes) std::memcpy(image.data() + at, v.data(), bytes);
+    // every table in one device allocation (256-byte aligned parts): the orbit and
+    // its events come from the host in one copy, the rest from k_orbit_tables
+    size_t bytes = 0;
+    auto part = [&bytes, count](size_t entry) -> size_t {
+        const size_t at = bytes;
+        bytes += (count * entry + 255) & ~(size_t)255;
         return at;
     };
-    const size_t at_z64 = stage(z64), at_z32 = stage(z32), at_z2 = stage(z2), at_bla16 = stage(bla16),
-                 at_bla64 = stage(bla64), at_lim = stage(lin_lim), at_ev = stage(next_event),
-                 at_bla16d = stage(bla16d), at_bla64d = stage(bla64d), at_limd = stage(lin_limd),
-                 at_z2_64 = stage(z2_64), at_ev64 = stage(next_event64);
+    const size_t at_z64 = part(16), at_ev = part(4), at_ev64 = part(4), sent = bytes;
+    const size_t at_z32 = part(8), at_z2 = part(8), at_z2_64 = part(16), at_bla16 = part(16), at_bla64 = part(16),
+                 at_bla16d = part(32), at_bla64d = part(32), at_lim = part(2), at_limd = part(2);
+    std::vector<unsigned char> image(sent);
+    std::memcpy(image.data() + at_z64, z64.data(), count * 16);
+    std::memcpy(image.data() + at_ev, next_event.data(), count * 4);
+    std::memcpy(image.data() + at_ev64, next_event64.data(), count * 4);
     unsigned char *dev = nullptr;
-    cudaError_t e = cudaMalloc(&dev, image.size());
-    if (e == cudaSuccess) e = cudaMemcpy(dev, image.data(), image.size(), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMalloc(&dev, bytes);
+    if (e == cudaSuccess) e = cudaMemcpy(dev, image.data(), sent, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        o->z64 = reinterpret_cast<double2 *>(dev + at_z64);
+        o->z32 = reinterpret_cast<float2 *>(dev + at_z32);
+        o->z2 = reinterpret_cast<float2 *>(dev + at_z2);
+        o->bla16 = reinterpret_cast<float4 *>(dev + at_bla16);
+        o->bla64 = reinterpret_cast<float4 *>(dev + at_bla64);
+        o->lin_lim = reinterpret_cast<char2 *>(dev + at_lim);
+        o->next_event = reinterpret_cast<uint32_t *>(dev + at_ev);
+        o->bla16d = reinterpret_cast<double2 *>(dev + at_bla16d);
+        o->bla64d = reinterpret_cast<double2 *>(dev + at_bla64d);
+        o->lin_limd = reinterpret_cast<char2 *>(dev + at_limd);
+        o->z2_64 = reinterpret_cast<double2 *>(dev + at_z2_64);
+        o->next_event64 = reinterpret_cast<uint32_t *>(dev + at_ev64);
+        const OrbitTables t{o->z64,   (uint32_t)count, o->z32,    o->z2,     o->z2_64,   o->bla16,
+                            o->bla64, o->lin_lim,      o->bla16d, o->bla64d, o->lin_limd};
+        // on the copy's stream; waited for, since the orbit may be used on any other
+        const dim3 grid((unsigned)((count + TABLE_THREADS - 1) / TABLE_THREADS), 2);
+        k_orbit_tables<<<grid, TABLE_THREADS>>>(t);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    }
     if (e != cudaSuccess) {
         if (dev) cudaFree(dev);
         delete o;
         return api_fail(CHAOS_ERR_CUDA, "reference orbit upload: %s", cudaGetErrorString(e));
     }
     o->arena = dev;
-    o->z64 = reinterpret_cast<double2 *>(dev + at_z64);
-    o->z32 = reinterpret_cast<float2 *>(dev + at_z32);
-    o->z2 = reinterpret_cast<float2 *>(dev + at_z2);
-    o->bla16 = reinterpret_cast<float4 *>(dev + at_bla16);
-    o->bla64 = reinterpret_cast<float4 *>(dev + at_bla64);
-    o->lin_lim = reinterpret_cast<char2 *>(dev + at_lim);
-    o->next_event = reinterpret_cast<uint32_t *>(dev + at_ev);
-    o->bla16d = reinterpret_cast<double2 *>(dev + at_bla16d);
-    o->bla64d = reinterpret_cast<double2 *>(dev + at_bla64d);
-    o->lin_limd = reinterpret_cast<char2 *>(dev + at_limd);
-    o->z2_64 = reinterpret_cast<double2 *>(dev + at_z2_64);
-    o->next_event64 = reinterpret_cast<uint32_t *>(dev + at_ev64);
     *out = o;
     return CHAOS_OK;
 }
