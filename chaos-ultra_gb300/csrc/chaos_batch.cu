@@ -63,6 +63,7 @@ template <> struct Num<float> {
     static __device__ __forceinline__ T zero() { return 0.f; }
     static __device__ __forceinline__ void step(T &x, T &y, T cx, T cy) { chaos::step<float, ARITH_FMA>(x, y, cx, cy); }
     static __device__ __forceinline__ float r2(T x, T y) { return radius2<float, ARITH_FMA>(x, y); }
+    static __device__ __forceinline__ bool below(T x, T y) { return below_four<ARITH_FMA>(x, y); }
     static __device__ __forceinline__ bool blockable(T cx, T cy) { return blockable_c(cx, cy); }
     static __device__ __forceinline__ bool interior(T cx, T cy) { return interior_c(cx, cy); }
 };
@@ -72,6 +73,7 @@ template <> struct Num<double> {
     static __device__ __forceinline__ T zero() { return 0.0; }
     static __device__ __forceinline__ void step(T &x, T &y, T cx, T cy) { chaos::step<double, ARITH_FMA>(x, y, cx, cy); }
     static __device__ __forceinline__ double r2(T x, T y) { return radius2<double, ARITH_FMA>(x, y); }
+    static __device__ __forceinline__ bool below(T x, T y) { return below_four<ARITH_FMA>(x, y); }
     static __device__ __forceinline__ bool blockable(T cx, T cy) { return blockable_c(cx, cy); }
     static __device__ __forceinline__ bool interior(T cx, T cy) { return interior_c(cx, cy); }
 };
@@ -98,6 +100,7 @@ template <> struct Num<R64> {
         chaos::step<double, ARITH_PARITY>(x, y, cx, cy);
     }
     static __device__ __forceinline__ double r2(T x, T y) { return radius2<double, ARITH_PARITY>(x, y); }
+    static __device__ __forceinline__ bool below(T x, T y) { return below_four<ARITH_PARITY>(x, y); }
     static __device__ __forceinline__ bool blockable(T cx, T cy) { return blockable_c(cx, cy); }
     static __device__ __forceinline__ bool interior(T cx, T cy) { return interior_c(cx, cy); }
 };
@@ -305,9 +308,7 @@ template <class N, int K> __global__ void __launch_bounds__(512) k_batch(BatchAr
             } else {
                 run_block([&](T &u, T &v) { P::step(u, v, cx, cy); });
             }
-            auto rr = P::r2(x, y);
-            r2 = (float)rr;
-            if (rr < 4) {
+            if (P::below(x, y)) {
                 const bool full = window == 0u && lim == (uint32_t)K;  // a checkpoint every K steps
                 i += lim;
                 window = window > 1u ? window - lim : 0u;
@@ -318,6 +319,7 @@ template <class N, int K> __global__ void __launch_bounds__(512) k_batch(BatchAr
                 if (i == max_iter) done = true;
             } else if (lim == 1u) {
                 i += 1u;
+                r2 = (float)P::r2(x, y);
                 done = true;
             } else {
                 x = sx;

@@ -151,6 +151,27 @@ template <class R, int A> __device__ __forceinline__ R radius2(R x, R y)
     return O::fma(x, x, O::mul(y, y));
 }
 
+// A binary64 as a binary32 on the integer units, truncated to 23 bits (0
+// below 2^-122, infinite from 2^117 on and for a NaN)
+__device__ __forceinline__ float float_of(double d)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(d), mag = hi & 0x7fffffffu;
+    const uint32_t f = (__funnelshift_l((uint32_t)__double2loint(d), hi, 3) & 0x7fffffffu) ^ 0x40000000u;
+    return __uint_as_float((hi & 0x80000000u) | (mag < (901u << 20) ? 0u : mag < (1140u << 20) ? f : 0x7f800000u));
+}
+
+// |z|^2 < 4 as radius2 tests it.  Binary64: in binary32 where that is clear
+// (float_of loses 2^-23 of each coordinate, 2^-21 of |z|^2 at most), which
+// leaves the binary64 pipe, the bound of every binary64 loop, its three
+// operations and the compare.
+template <int A> __device__ __forceinline__ bool below_four(float x, float y) { return radius2<float, A>(x, y) < 4.f; }
+template <int A> __device__ __forceinline__ bool below_four(double x, double y)
+{
+    const float fx = float_of(x), fy = float_of(y);
+    if (fmaf(fx, fx, fy * fy) < 3.99f) return true;
+    return radius2<double, A>(x, y) < 4.0;
+}
+
 // One step of z <- z^2 + c.
 //   parity:     x' = (x*x - y*y) + cx, y' = (2*x)*y + cy  (mandelbrot.cu:17-18 order)
 //   contracted: x' as parity, y' = fma(x + x, y, cy)
@@ -394,7 +415,7 @@ __device__ __forceinline__ uint32_t escape(uint32_t max_iter, R x, R y, R cx, R 
 #pragma unroll
                 for (int k = 0; k < ESCAPE_BLOCK; k++) step<R, A>(x, y, cx, cy);
             }
-            if (!(radius2<R, A>(x, y) < R(4))) {
+            if (!below_four<A>(x, y)) {
                 x = sx;
                 y = sy;
                 break;

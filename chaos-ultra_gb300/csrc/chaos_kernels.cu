@@ -24,6 +24,51 @@ namespace chaos {
 constexpr uint32_t PALETTE_SMEM = 4096;
 
 // ---------------------------------------------------------------------------
+// Packing a block's working lanes into as few warps as hold them
+// ---------------------------------------------------------------------------
+
+template <class S> constexpr uint32_t LANE_WORDS = (uint32_t)(sizeof(S) / 4);
+
+// All threads of the block take part.  `left` is the number of lanes at work
+// that the caller packed for last (the block's threads at first) and becomes
+// their number now; the states move only where that saves a warp.  `keep`:
+// this lane is at work; on return `on` says so of the lane's new state.
+// buf holds LANE_WORDS<S> words a thread, count one a warp.
+template <class S>
+__device__ __forceinline__ void pack_lanes(S &st, bool keep, bool &on, uint32_t &left, uint32_t *buf, uint32_t *count)
+{
+    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const uint32_t mask = __ballot_sync(FULL, keep);
+    __syncthreads();  // the last packing's words and counts have been read
+    if (lane == 0) count[wib] = (uint32_t)__popc(mask);
+    __syncthreads();
+    uint32_t at = (uint32_t)__popc(mask & ((1u << lane) - 1u)), now = 0;
+    for (uint32_t k = 0; k < warps; k++) {
+        const uint32_t c = count[k];
+        at += k < wib ? c : 0u;
+        now += c;
+    }
+    const bool pack = (now + 31u) / 32u < (left + 31u) / 32u;
+    left = now;
+    on = keep;
+    if (!pack) return;
+    constexpr uint32_t W = LANE_WORDS<S>;
+    uint32_t words[W];
+    if (keep) {
+        memcpy(words, &st, sizeof(S));
+#pragma unroll
+        for (uint32_t k = 0; k < W; k++) buf[k * blockDim.x + at] = words[k];
+    }
+    __syncthreads();
+    on = threadIdx.x < now;
+    if (on) {
+#pragma unroll
+        for (uint32_t k = 0; k < W; k++) words[k] = buf[k * blockDim.x + threadIdx.x];
+        memcpy(&st, words, sizeof(S));
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Independent-sample frames with per-lane refill
 // ---------------------------------------------------------------------------
 
@@ -45,11 +90,29 @@ __device__ __forceinline__ void frame_point(const FrameArgs<R> &a, uint32_t w_ma
     cy = O::fma(-dyp, a.ps, a.center_y);
 }
 
+// Binary64 frames.  Bound: the binary64 pipe (a warp's operation takes its
+// scheduler's pipe 76 cycles; five operations a step rounded, three fused).
+// Once the pixels are claimed the remaining lanes are packed: 640x360 pixels of
+// 4 samples at span 1.7e-8, maxIter 20000, are 1.5 pixels a lane and took 222 ms
+// with the lanes left where they were, 175 packed and 172 with the clear escape
+// tests in binary32 (480x270: 115 -> 99 ms); 512-step epochs, 128 and 2048 steps
+// gave 175 and 180, three or four blocks an SM (80 and 64 registers) 176 and 185.
+constexpr int DRAIN_ROUNDS = 32;  // rounds between packings
+struct FrameLane {
+    double x, y, cx, cy;
+    CycleWatch<double> cw;
+    uint32_t pix, s, i, window;
+    float acc_v, acc[4];
+    bool blk, begin;
+};
+
 template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_frame(FrameArgs<double> a)
 {
     using R = double;
     constexpr int K = ESCAPE_BLOCK;
     __shared__ uint32_t s_pal[PALETTE_SMEM];
+    __shared__ uint32_t s_state[LANE_WORDS<FrameLane> * PERSIST_THREADS], s_count[PERSIST_THREADS / 32], s_drain;
+    if (threadIdx.x == 0) s_drain = 0;
     const uint32_t *pal = a.palette;
     if (a.rgba && a.palette_len <= PALETTE_SMEM) {
         for (uint32_t k = threadIdx.x; k < a.palette_len; k += blockDim.x) s_pal[k] = a.palette[k];
@@ -60,53 +123,86 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     const uint32_t w_magic = div_magic(a.w);
-    uint32_t pix = 0xffffffffu, s = 0, i = 0;
-    R x = R(0), y = R(0), cx = R(0), cy = R(0);
-    bool blk = false, need = true, begin = false;
-    uint32_t window = 0;  // > 0: the escape lies within the next `window` steps
-    float acc_v = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+    FrameLane st{};
+    R &x = st.x, &y = st.y, &cx = st.cx, &cy = st.cy;
+    CycleWatch<R> &cw = st.cw;  // exact cycle detection (see CycleWatch)
+    uint32_t &pix = st.pix, &s = st.s, &i = st.i;
+    uint32_t &window = st.window;  // > 0: the escape lies within the next `window` steps
+    float &acc_v = st.acc_v, (&acc)[4] = st.acc;
+    pix = 0xffffffffu;
+    bool need = true;
     unsigned long long iters = 0, skipped = 0;
-    CycleWatch<R> cw;  // exact cycle detection (see CycleWatch)
     const unsigned long long t_start = a.budget_ns ? global_ns() : 0ull;
 
-    // the grid's first pixels go out without a claim (warp w takes 32w..32w+31),
-    // so the launch does not start with every warp's atomic on one counter;
-    // claims then count from there
+    // the grid's first pixels go out without a claim (32 to a warp, neighbouring
+    // ones to different blocks), so the launch does not start with every warp's
+    // atomic on one counter; claims then count from there
     const uint32_t n_warps = gridDim.x * (blockDim.x >> 5);
     bool first = true;
 
+    // Two phases, one loop.  First every lane whose pixel is complete takes the
+    // next one.  Once the pixels are gone for one of the block's warps (s_drain)
+    // the lanes still at work are packed into as few warps as hold them, again
+    // and again as they end: a warp's step takes the binary64 pipe the same time
+    // with one lane as with 32, and a pixel runs for up to samples x maxIterations
+    // steps.
+    bool drain = false, on = true;
+    uint32_t left = blockDim.x, rounds = 0;
     for (;;) {
         // a time limit: the warp stops where it is (its samples in flight stay unwritten)
-        if (out_of_time(a.budget_ns, t_start, a.status, lane)) break;
-        uint32_t need_mask = __ballot_sync(FULL, need);
-        if (need_mask) {
-            uint32_t base = 0;
-            if (first) {
-                base = 32u * (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
-                first = false;
-            } else {
-                const uint32_t leader = __ffs(need_mask) - 1u;
-                if (lane == leader) base = 32u * n_warps + atomicAdd(a.counter, (uint32_t)__popc(need_mask));
-                base = __shfl_sync(FULL, base, leader);
+        const bool late = out_of_time(a.budget_ns, t_start, a.status, lane);
+        if (!drain) {
+            const uint32_t need_mask = __ballot_sync(FULL, need);
+            if (need_mask && !late) {
+                uint32_t base = 0;
+                if (first) {
+                    base = 32u * ((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+                    first = false;
+                } else {
+                    const uint32_t leader = __ffs(need_mask) - 1u;
+                    if (lane == leader) base = 32u * n_warps + atomicAdd(a.counter, (uint32_t)__popc(need_mask));
+                    base = __shfl_sync(FULL, base, leader);
+                }
+                if (need) {
+                    pix = base + (uint32_t)__popc(need_mask & lt_mask);
+                    need = false;
+                    st.begin = true;
+                    s = 0;
+                    acc_v = 0.f;
+                    acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+                }
             }
-            if (need) {
-                pix = base + (uint32_t)__popc(need_mask & lt_mask);
+            if (late || __any_sync(FULL, pix >= a.n_pix)) {
+                if (lane == 0) *(volatile uint32_t *)&s_drain = 1;
+                drain = true;
+            } else {
+                drain = *(volatile uint32_t *)&s_drain != 0;
+            }
+            on = !need && pix < a.n_pix;
+            rounds = 0;
+        }
+        if (drain) {
+            on = on && !need && !late;
+            if (rounds == 0) {
+                pack_lanes(st, on, on, left, s_state, s_count);
+                if (left == 0) break;
                 need = false;
-                begin = true;
-                s = 0;
-                acc_v = 0.f;
-                acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+                rounds = DRAIN_ROUNDS;
+            }
+            --rounds;
+            if (!__any_sync(FULL, on)) {
+                rounds = 0;  // to the next packing
+                continue;
             }
         }
-        const bool active = pix < a.n_pix;
-        if (!__any_sync(FULL, active)) break;
+        const bool active = on;
 
         bool done = false;
         R r2 = R(0);
         uint32_t lim = 0;  // steps this lane takes this round: a power of two <= K
         if (active) {
-            if (begin) {
-                begin = false;
+            if (st.begin) {
+                st.begin = false;
                 R px, py;
                 frame_point(a, w_magic, pix, s, px, py);
                 i = 0;
@@ -129,7 +225,7 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
                     cx = a.jcx;
                     cy = a.jcy;
                 }
-                blk = blockable_c(cx, cy);
+                st.blk = blockable_c(cx, cy);
                 window = 0;
                 cw.reset(x, y);
                 r2 = radius2<R, A>(x, y);
@@ -142,7 +238,7 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
                 }
             }
             if (!done) {
-                if (!blk) {
+                if (!st.blk) {
                     lim = 1;
                 } else if (window) {
                     lim = window > 1u ? window >> 1 : 1u;
@@ -202,8 +298,7 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
                     run_block([&](R &u, R &v) { step<R, A>(u, v, cx, cy); });
                 }
             }
-            r2 = radius2<R, A>(x, y);
-            if (r2 < R(4)) {
+            if (below_four<A>(x, y)) {
                 const bool full = window == 0u && lim == (uint32_t)K;  // a checkpoint every K steps
                 i += lim;
                 window = window > 1u ? window - lim : 0u;
@@ -214,6 +309,7 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
                 if (i == a.max_iter) done = true;
             } else if (lim == 1u) {
                 i += 1u;  // the escape step
+                r2 = radius2<R, A>(x, y);
                 done = true;
             } else {
                 // the escape lies within these lim steps: search them
@@ -252,7 +348,7 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
                 if (a.rgba) a.rgba[pix] = frame_pack_rgba(acc, a.spp);
                 need = true;
             } else {
-                begin = true;
+                st.begin = true;
             }
         }
     }
@@ -746,7 +842,13 @@ template <int A, int F> static cudaError_t launch_frame64(const FrameArgs<double
 {
     static const int occ = occupancy(k_frame<A, F>, PERSIST_THREADS);
     unsigned long long warps = ((unsigned long long)a.n_pix + 31ull) / 32ull;
-    k_frame<A, F><<<grid_for(warps, occ, sms), PERSIST_THREADS, 0, s>>>(a);
+    // frames of fewer warps than eight an SM spread over all SMs (each has its own
+    // binary64 pipe) in smaller blocks
+    const unsigned long long per_sm = (warps + (unsigned)sms - 1ull) / (unsigned)sms;
+    const unsigned threads = per_sm >= PERSIST_THREADS / 32 ? PERSIST_THREADS : 32u * (unsigned)per_sm;
+    const unsigned long long blocks = (warps + threads / 32u - 1ull) / (threads / 32u);
+    const unsigned grid = (unsigned)std::min(blocks, (unsigned long long)occ * (unsigned)sms);
+    k_frame<A, F><<<grid, threads, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -158,15 +158,6 @@ __device__ __forceinline__ double double_of(int k)
     return __dsub_rn(__hiloint2double(0x43300000, k ^ (int)0x80000000), 4503601774854144.0);
 }
 
-// A binary64 as a binary32 on the integer units, truncated to 23 bits (0
-// below 2^-122, infinite from 2^117 on and for a NaN)
-__device__ __forceinline__ float float_of(double d)
-{
-    const uint32_t hi = (uint32_t)__double2hiint(d), mag = hi & 0x7fffffffu;
-    const uint32_t f = (__funnelshift_l((uint32_t)__double2loint(d), hi, 3) & 0x7fffffffu) ^ 0x40000000u;
-    return __uint_as_float((hi & 0x80000000u) | (mag < (901u << 20) ? 0u : mag < (1140u << 20) ? f : 0x7f800000u));
-}
-
 // 2^e as a binary32, or 0 below the normal range
 __device__ __forceinline__ float pow2f(int e) { return e >= -126 ? __int_as_float((e + 127) << 23) : 0.f; }
 
