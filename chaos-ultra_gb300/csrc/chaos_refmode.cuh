@@ -5,6 +5,7 @@
 // modules) and chaos_newton.cu (Newton modules, built without contraction).
 #pragma once
 
+#include "chaos_claim.cuh"
 #include "chaos_kernels.cuh"
 
 namespace chaos {
@@ -48,6 +49,18 @@ __device__ __forceinline__ void for_each_strip(uint32_t *counter, uint32_t n_til
         if (size == 1u && lane == 0) claim = atomicAdd(counter, next);
         t0 = __shfl_sync(FULL, claim, 0);
         size = next;
+    }
+}
+
+// The same with strips of up to `strip` tiles from the block's pieces, each
+// taken when it is needed.
+template <class Body> __device__ __forceinline__ void for_each_claim(Claims &claims, uint32_t strip, Body body)
+{
+    for (;;) {
+        uint32_t got;
+        const uint32_t t0 = claims.take(strip, got);
+        if (got == 0u) break;
+        body(t0, t0 + got);
     }
 }
 
@@ -113,6 +126,8 @@ template <class R, int A, int F> __global__ void __launch_bounds__(PERSIST_THREA
     add_total(a.total, iters, lane);
 }
 
+constexpr uint32_t PIECE_TILES = 4 * PERSIST_THREADS / 32;  // a group of four for each warp
+
 // Tiles whose previous-frame reads are in flight together.  A reuse-dominated
 // frame is a stream of small dependent steps per tile (origin -> four loads
 // -> filter -> store); with one tile's loads in flight per warp and the
@@ -176,7 +191,7 @@ __device__ __forceinline__ void advanced_strip(const AdvancedArgs<R> &a, const S
             const bool valid = p.x < a.m.size.x && p.y < a.m.size.y;
             const float2 vw = reuse ? stage[32u * row + 8u * k + col] : make_float2(0.f, 0.f);
             const bool reusing = valid && reuse && !(vw.y < 0.1f);
-            if (!fov && __all_sync(FULL, reusing || !valid)) {
+            if ((!fov || clear_of_fovea(a.focus, x0, y0)) && __all_sync(FULL, reusing || !valid)) {
                 // every pixel reuses and none takes new samples: the record is
                 // (value, weight, isReused = 1, 0), as the full path stores it
                 if (valid) {
@@ -193,7 +208,15 @@ __device__ __forceinline__ void advanced_strip(const AdvancedArgs<R> &a, const S
     }
 }
 
-template <class R, int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_advanced(AdvancedArgs<R> a)
+// PIECES: strips of one group from 32-tile pieces that a block claims, for large
+// frames with a foveal region, whose tiles take samples: guided strips of up to
+// 16 tiles gave one warp that many of them, and single groups from the one
+// counter are 65,000 claims of 2 ns.  3840x2160, zooming in: 142 -> 112 us.  A
+// resting 7680x4320 frame takes 209 us with guided strips and 240 with pieces
+// (64- and 128-tile pieces 268 and 276, guided strips of up to 32 tiles 235: the
+// longer a warp's strip, the wider the band of rows that is read at a time).
+template <class R, int A, int F, bool PIECES>
+__global__ void __launch_bounds__(PERSIST_THREADS) k_advanced(AdvancedArgs<R> a)
 {
     const uint32_t lane = threadIdx.x & 31u;
     SampleGeometry<R> g = make_geometry(a.m.image, a.m.size, a.m.max_iter, a.m.jcx, a.m.jcy);
@@ -202,14 +225,20 @@ template <class R, int A, int F> __global__ void __launch_bounds__(PERSIST_THREA
     __shared__ float2 s_stage[PERSIST_THREADS / 32][4 * 32];
     float2 *stage = s_stage[threadIdx.x >> 5];
     const bool al8 = ((reinterpret_cast<uintptr_t>(a.in) | (uintptr_t)a.in_pitch) & 7u) == 0;
-    if (al8)
-        for_each_strip(a.m.counter, a.m.n_tiles, a.m.tile_chunk, lane, [&](uint32_t t0, uint32_t t1) {
-            advanced_strip<R, A, F, true>(a, g, lane, stage, t0, t1, iters);
-        });
+    auto each = [&](auto strip) {
+        if constexpr (PIECES) {
+            __shared__ ClaimShared s_claims;
+            Claims claims(s_claims, a.m.counter, ClaimPlan{a.m.n_tiles, PIECE_TILES});
+            __syncthreads();
+            for_each_claim(claims, 4u, strip);
+        } else {
+            for_each_strip(a.m.counter, a.m.n_tiles, a.m.tile_chunk, lane, strip);
+        }
+    };
+    if (PIECES || al8)
+        each([&](uint32_t t0, uint32_t t1) { advanced_strip<R, A, F, true>(a, g, lane, stage, t0, t1, iters); });
     else
-        for_each_strip(a.m.counter, a.m.n_tiles, a.m.tile_chunk, lane, [&](uint32_t t0, uint32_t t1) {
-            advanced_strip<R, A, F, false>(a, g, lane, stage, t0, t1, iters);
-        });
+        each([&](uint32_t t0, uint32_t t1) { advanced_strip<R, A, F, false>(a, g, lane, stage, t0, t1, iters); });
     add_total(a.m.total, iters, lane);
 }
 
@@ -241,11 +270,23 @@ template <class R, int A, int F> static cudaError_t launch_main_t(const MainArgs
 template <class R, int A, int F>
 static cudaError_t launch_advanced_t(const AdvancedArgs<R> &args, int sms, cudaStream_t s)
 {
-    static const int occ = occupancy(k_advanced<R, A, F>, PERSIST_THREADS);
+    static const int occ = occupancy(k_advanced<R, A, F, false>, PERSIST_THREADS);
     AdvancedArgs<R> a = args;
     a.m.tile_chunk = tile_chunk_for(a.m.n_tiles, occ, sms);
-    k_advanced<R, A, F><<<grid_for((a.m.n_tiles + a.m.tile_chunk - 1) / a.m.tile_chunk, occ, sms), PERSIST_THREADS, 0,
-                          s>>>(a);
+    if constexpr (sizeof(R) == 4 && F <= FRACTAL_JULIA) {
+        // where guided strips would hold whole groups (smaller frames go tile by
+        // tile), and the previous frame's pairs can be read 8 bytes at a time
+        const bool fov =
+            (a.m.flags & FLAG_FOVEATION) && (a.m.flags & FLAG_IS_ZOOMING) && (a.m.flags & FLAG_ZOOMING_IN);
+        const bool al8 = ((reinterpret_cast<uintptr_t>(a.in) | (uintptr_t)a.in_pitch) & 7u) == 0;
+        if (fov && al8 && a.m.tile_chunk >= 4u) {
+            static const int occ_p = occupancy(k_advanced<R, A, F, true>, PERSIST_THREADS);
+            k_advanced<R, A, F, true><<<grid_for((a.m.n_tiles + 3u) / 4u, occ_p, sms), PERSIST_THREADS, 0, s>>>(a);
+            return cudaGetLastError();
+        }
+    }
+    k_advanced<R, A, F, false><<<grid_for((a.m.n_tiles + a.m.tile_chunk - 1) / a.m.tile_chunk, occ, sms),
+                                 PERSIST_THREADS, 0, s>>>(a);
     return cudaGetLastError();
 }
 
