@@ -56,9 +56,10 @@ int cuda_fail(cudaError_t e, const char *what)
     } while (0)
 
 // Per-device state: SM count and a ring of work counters.  Each persistent
-// launch takes the next slot and zeroes it on its own stream first, so
-// launches in flight on different streams use different counters (up to
-// kCounterSlots of them at once).
+// launch takes the next slot, so launches in flight on different streams use
+// different counters (up to kCounterSlots of them at once).  A slot is a work
+// counter and its companion (zero between launches: the kernels leave them so,
+// see leave_counter) and a status word.
 constexpr int kMaxDevices = 64;
 constexpr uint32_t kCounterSlots = 4096;
 
@@ -79,7 +80,10 @@ int device_state(DeviceState **out)
     DeviceState &d = g_devices[dev];
     std::call_once(d.once, [&]() {
         cudaError_t e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess) e = cudaMalloc(&d.counters, 2 * kCounterSlots * sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaMalloc(&d.counters, 3 * kCounterSlots * sizeof(uint32_t));
+        // (on the legacy stream, and waited for: the first launch may be on any other)
+        if (e == cudaSuccess) e = cudaMemset(d.counters, 0, 3 * kCounterSlots * sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
         d.init_error = e;
     });
     if (d.init_error != cudaSuccess) return cuda_fail(d.init_error, "device set-up");
@@ -87,12 +91,11 @@ int device_state(DeviceState **out)
     return CHAOS_OK;
 }
 
-int take_counter(DeviceState *d, cudaStream_t s, uint32_t **counter)
+void take_counter(DeviceState *d, uint32_t **counter, uint32_t **done)
 {
     uint32_t slot = d->next.fetch_add(1, std::memory_order_relaxed) % kCounterSlots;
     *counter = d->counters + slot;
-    CHAOS_CUDA(cudaMemsetAsync(*counter, 0, sizeof(uint32_t), s), "cudaMemsetAsync(work counter)");
-    return CHAOS_OK;
+    *done = d->counters + 2 * kCounterSlots + slot;
 }
 
 // The status word that goes with a counter slot (a launch with a time limit
@@ -306,13 +309,14 @@ int api_fail(int code, const char *fmt, ...)
     return code;
 }
 
-int api_device_counter(cudaStream_t s, uint32_t **counter, int *sms)
+int api_device_counter(uint32_t **counter, uint32_t **done, int *sms)
 {
     DeviceState *d;
     int rc = device_state(&d);
     if (rc) return rc;
     *sms = d->sms;
-    return take_counter(d, s, counter);
+    take_counter(d, counter, done);
+    return CHAOS_OK;
 }
 
 int api_device_status(const uint32_t *counter, cudaStream_t s, uint32_t **status)
@@ -524,7 +528,7 @@ static int render_main(chaos_module *m, chaos_pixel_info *out, long pitch, uint3
     a.newton = m->newton;
     a.tiles_x = (w + 7u) / 8u;
     a.n_tiles = a.tiles_x * ((h + 3u) / 4u);
-    if ((rc = take_counter(d, s, &a.counter))) return rc;
+    take_counter(d, &a.counter, &a.done);
     return finish(launch_main<R>(a, arith_of(arith), m->fractal, d->sms, s), s, sync);
 }
 
@@ -566,7 +570,7 @@ static int render_advanced(chaos_module *m, chaos_pixel_info *out, long pitch, u
     a.in = in;
     a.in_pitch = in_pitch;
     a.focus = UInt2{fx, fy};
-    if ((rc = take_counter(d, s, &a.m.counter))) return rc;
+    take_counter(d, &a.m.counter, &a.m.done);
     return finish(launch_advanced<R>(a, arith_of(arith), m->fractal, d->sms, s), s, sync);
 }
 
@@ -718,7 +722,7 @@ static int frame_impl(const chaos_frame_desc *dsc, const chaos_frame_out *o, cud
     a.total = o->total_iterations;
     a.skipped = o->cycle_skipped;
     budget_of(dsc->time_limit_s, &a.budget_ns);
-    if ((rc = take_counter(d, s, &a.counter))) return rc;
+    take_counter(d, &a.counter, &a.done);
     a.status = o->status;
     if (a.budget_ns && !a.status) {
         if (!sync && !status_used)

@@ -16,6 +16,21 @@
 
 namespace chaos {
 
+// The end of a persistent kernel: the launch's last warp leaves the work counter
+// at zero for the launch that takes it next (a memset before every launch cost
+// a small frame as much as its kernel).  Each warp's lane 0 calls it after the
+// warp's last claim.  retired: shared, zero from before the block's first
+// barrier; done: the counter's companion word, zero between launches, or null
+// where the caller zeroes the counter.
+__device__ __forceinline__ void leave_counter(uint32_t *counter, uint32_t *done, uint32_t *retired)
+{
+    if (!done) return;
+    if (atomicAdd(retired, 1u) + 1u != (blockDim.x >> 5)) return;
+    if (atomicAdd(done, 1u) + 1u != gridDim.x) return;
+    *counter = 0u;
+    *done = 0u;
+}
+
 // Pieces of `size` items; the first of every block goes out without a claim
 // (block b has [b size, (b + 1) size)).
 struct ClaimPlan {

@@ -111,8 +111,8 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
     using R = double;
     constexpr int K = ESCAPE_BLOCK;
     __shared__ uint32_t s_pal[PALETTE_SMEM];
-    __shared__ uint32_t s_state[LANE_WORDS<FrameLane> * PERSIST_THREADS], s_count[PERSIST_THREADS / 32], s_drain;
-    if (threadIdx.x == 0) s_drain = 0;
+    __shared__ uint32_t s_state[LANE_WORDS<FrameLane> * PERSIST_THREADS], s_count[PERSIST_THREADS / 32], s_drain, s_retired;
+    if (threadIdx.x == 0) s_drain = s_retired = 0;
     const uint32_t *pal = a.palette;
     if (a.rgba && a.palette_len <= PALETTE_SMEM) {
         for (uint32_t k = threadIdx.x; k < a.palette_len; k += blockDim.x) s_pal[k] = a.palette[k];
@@ -362,6 +362,7 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
         for (int o = 16; o > 0; o >>= 1) skipped += __shfl_down_sync(FULL, skipped, o);
         if (lane == 0 && skipped) atomicAdd(a.skipped, skipped);
     }
+    if (lane == 0) leave_counter(a.counter, a.done, &s_retired);
 }
 
 // ---------------------------------------------------------------------------
@@ -408,7 +409,8 @@ __global__ void __launch_bounds__(frame32_threads<MULTI>()) k_frame32(FrameArgs<
     constexpr int WORDS = MULTI ? 12 : 6, WARPS = frame32_threads<MULTI>() / 32;
     __shared__ uint32_t s_pal[PALETTE_SMEM];
     __shared__ uint32_t s_queue[WARPS][WORDS][QUEUE];
-    __shared__ uint32_t s_count[WARPS];
+    __shared__ uint32_t s_count[WARPS], s_retired;
+    if (threadIdx.x == 0) s_retired = 0;
     const uint32_t *pal = a.palette;
     if (a.rgba && a.palette_len <= PALETTE_SMEM) {
         for (uint32_t k = threadIdx.x; k < a.palette_len; k += blockDim.x) s_pal[k] = a.palette[k];
@@ -741,6 +743,7 @@ __global__ void __launch_bounds__(frame32_threads<MULTI>()) k_frame32(FrameArgs<
         for (int o = 16; o > 0; o >>= 1) skipped += __shfl_down_sync(FULL, skipped, o);
         if (lane == 0 && skipped) atomicAdd(a.skipped, skipped);
     }
+    if (lane == 0) leave_counter(a.counter, a.done, &s_retired);
 }
 
 // ---------------------------------------------------------------------------

@@ -50,13 +50,14 @@
 
 #include "../../include/chaos_gb300.h"
 #include "bigfix.h"
+#include "chaos_claim.cuh"
 #include "chaos_kernels.cuh"
 #include "chaos_trace.h"
 
 namespace chaos {
 
 int api_fail(int code, const char *fmt, ...);  // chaos_api.cu
-int api_device_counter(cudaStream_t s, uint32_t **counter, int *sms);
+int api_device_counter(uint32_t **counter, uint32_t **done, int *sms);
 int api_device_status(const uint32_t *counter, cudaStream_t s, uint32_t **status);
 bool api_budget(double seconds, unsigned long long *ns);
 int api_read_status(const uint32_t *status, cudaStream_t s, double seconds);
@@ -98,7 +99,7 @@ template <class D> struct PerturbArgs {
     uint32_t interior_rgba;
     unsigned long long *total;
     unsigned long long *rebases;
-    uint32_t *counter;
+    uint32_t *counter, *done;      // see leave_counter
     unsigned long long budget_ns;  // 0, or the run time after which warps stop (RUN_STATUS_TIMEOUT into *status)
     uint32_t *status;
     // binary32 set-up of rescaled samples at pixel centres (dc_fast): with
@@ -197,7 +198,8 @@ template <class D, int K, bool S> __global__ void __launch_bounds__(256, sizeof(
     static_assert(!S || sizeof(D) == 4, "rescaling is for binary32 differences");
     using O = Op<D>;
     constexpr uint32_t FULLM = 0xffffffffu;
-    __shared__ uint32_t s_pal[4096];
+    __shared__ uint32_t s_pal[4096], s_retired;
+    if (threadIdx.x == 0) s_retired = 0;
     const uint32_t *pal = a.palette;
     if (a.rgba && a.palette_len <= 4096u) {
         for (uint32_t k = threadIdx.x; k < a.palette_len; k += blockDim.x) s_pal[k] = a.palette[k];
@@ -368,6 +370,35 @@ template <class D, int K, bool S> __global__ void __launch_bounds__(256, sizeof(
                     // plain difference too large for them): plain steps for the rest of
                     // the round.  Taken by the whole group only: a lane that entered
                     // alone would run its loop while the others wait, and then they theirs.
+                    if constexpr (sizeof(D) == 4) {
+                        // binary32: neither the orbit's end nor the iteration limit comes
+                        // within the next n steps, so those run without their tests and
+                        // with the glitch test's two thresholds in one (|z|^2 below |d|^2,
+                        // or so small that the squares may have underflowed).
+                        // 1920x1080, span 1e-200: 166 -> 158 us.
+                        const uint32_t n = min((uint32_t)(K - k), min(a.max_iter - i, a.orbit_last - m) - 1u);
+                        const uint32_t end = m + n;
+                        uint32_t at = m;
+#pragma unroll 1
+                        while (at != end) {
+                            const D wx = O::fma(D(2), Zx, dx), wy = O::fma(D(2), Zy, dy);
+                            const D ndx = O::fma(wx, dx, O::fma(-wy, dy, dcx));
+                            const D ndy = O::fma(wx, dy, O::fma(wy, dx, dcy));
+                            const typename Vec2T<D>::type Z = a.orbit[at + 1u];
+                            const D zx = O::add(Z.x, ndx), zy = O::add(Z.y, ndy);
+                            r2 = O::fma(zx, zx, O::mul(zy, zy));
+                            const float d2 = __fmaf_rn((float)ndx, (float)ndx, __fmul_rn((float)ndy, (float)ndy));
+                            if (!(r2 < D(4)) || (float)r2 < fmaxf(d2, 0x1p-60f)) break;
+                            dx = ndx;
+                            dy = ndy;
+                            Zx = Z.x;
+                            Zy = Z.y;
+                            ++at;
+                        }
+                        i += at - m;
+                        k += (int)(at - m);  // (a step that a test stopped at is taken again below)
+                        m = at;
+                    }
 #pragma unroll 1
                     for (; k < K; k++)
                         if (plain_step()) {
@@ -636,6 +667,7 @@ template <class D, int K, bool S> __global__ void __launch_bounds__(256, sizeof(
     if (lane == 0) {
         if (a.total && iters) atomicAdd(a.total, iters);
         if (a.rebases && rebases) atomicAdd(a.rebases, rebases);
+        leave_counter(a.counter, a.done, &s_retired);
     }
 }
 
@@ -1052,7 +1084,7 @@ static int perturb_impl(const chaos_frame_desc *d, const chaos_orbit *orb, const
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     } else {
-        int rc = api_device_counter(s, &a.counter, &sms);
+        int rc = api_device_counter(&a.counter, &a.done, &sms);
         if (rc) return rc;
     }
     if (a.budget_ns && !a.status) {

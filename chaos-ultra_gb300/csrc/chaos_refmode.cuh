@@ -116,6 +116,9 @@ static inline uint32_t tile_chunk_for(uint32_t n_tiles, int occ, int sms, uint32
 
 template <class R, int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_main(MainArgs<R> a)
 {
+    __shared__ uint32_t s_retired;
+    if (threadIdx.x == 0) s_retired = 0;
+    __syncthreads();
     const uint32_t lane = threadIdx.x & 31u;
     SampleGeometry<R> g = make_geometry(a.image, a.size, a.max_iter, a.jcx, a.jcy);
     g.newton = a.newton;
@@ -124,6 +127,7 @@ template <class R, int A, int F> __global__ void __launch_bounds__(PERSIST_THREA
         render_main_tile<R, A, F>(g, a.out, a.pitch, a.size, x0, y0, lane, a.max_ss, a.flags, iters);
     });
     add_total(a.total, iters, lane);
+    if (lane == 0) leave_counter(a.counter, a.done, &s_retired);
 }
 
 constexpr uint32_t PIECE_TILES = 4 * PERSIST_THREADS / 32;  // a group of four for each warp
@@ -223,6 +227,9 @@ __global__ void __launch_bounds__(PERSIST_THREADS) k_advanced(AdvancedArgs<R> a)
     g.newton = a.m.newton;
     unsigned long long iters = 0;
     __shared__ float2 s_stage[PERSIST_THREADS / 32][4 * 32];
+    __shared__ uint32_t s_retired;
+    if (threadIdx.x == 0) s_retired = 0;
+    __syncthreads();
     float2 *stage = s_stage[threadIdx.x >> 5];
     const bool al8 = ((reinterpret_cast<uintptr_t>(a.in) | (uintptr_t)a.in_pitch) & 7u) == 0;
     auto each = [&](auto strip) {
@@ -240,6 +247,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS) k_advanced(AdvancedArgs<R> a)
     else
         each([&](uint32_t t0, uint32_t t1) { advanced_strip<R, A, F, false>(a, g, lane, stage, t0, t1, iters); });
     add_total(a.m.total, iters, lane);
+    if (lane == 0) leave_counter(a.m.counter, a.m.done, &s_retired);
 }
 
 template <class KernelPtr> static int occupancy(KernelPtr k, int threads)
