@@ -94,35 +94,27 @@ inline BigFix bigfix_neg(BigFix a)
 
 inline BigFix bigfix_sub(const BigFix &a, const BigFix &b) { return bigfix_add(a, bigfix_neg(b)); }
 
-// The product of a and b (limbs 0..L) without the limb products of the columns
-// below `first`, row by row into p[first..2L].
-inline void bigfix_rows(const uint64_t *a, const uint64_t *b, int L, int first, uint64_t *p)
-{
-    for (int c = first; c <= 2 * L + 1; c++) p[c] = 0;
-    for (int i = 0; i <= L; i++) {
-        uint64_t carry = 0;
-        const uint64_t x = a[i];
-        for (int j = first > i ? first - i : 0; j <= L; j++) {
-            const unsigned __int128 t = (unsigned __int128)x * b[j] + p[i + j] + carry;
-            p[i + j] = (uint64_t)t;
-            carry = (uint64_t)(t >> 64);
-        }
-        p[i + L + 1] = carry;  // the first row to reach this column
-    }
-}
-
-// a * b, truncated to L fraction limbs.  The result is columns L..2L of the
-// full product.  What the columns below L-2 would carry in is less than L at
-// column L-1, so unless that column's word is within L + 2 of overflowing, two
-// guard columns give the full product's words exactly; otherwise all columns
-// are formed.  (About half the limb products of the full one: an orbit step of
-// 1088 bits takes 0.45 us where it took 0.63 on a Grace core.)
+// a * b, truncated to L fraction limbs.
 inline BigFix bigfix_mul(const BigFix &a, const BigFix &b)
 {
-    const int L = a.limbs, first = L > 2 ? L - 2 : 0;
-    uint64_t p[2 * BIGFIX_MAX_LIMBS + 2];
-    bigfix_rows(a.w, b.w, L, first, p);
-    if (first > 0 && p[L - 1] >= ~(uint64_t)0 - (uint64_t)(L + 2)) bigfix_rows(a.w, b.w, L, 0, p);
+    const int L = a.limbs;
+    uint64_t p[2 * BIGFIX_MAX_LIMBS + 3] = {};
+    for (int i = 0; i <= L; i++) {
+        if (!a.w[i]) continue;
+        unsigned __int128 carry = 0;
+        for (int j = 0; j <= L; j++) {
+            unsigned __int128 t = (unsigned __int128)a.w[i] * b.w[j] + p[i + j] + carry;
+            p[i + j] = (uint64_t)t;
+            carry = t >> 64;
+        }
+        int k = i + L + 1;
+        while (carry) {
+            unsigned __int128 t = (unsigned __int128)p[k] + carry;
+            p[k] = (uint64_t)t;
+            carry = t >> 64;
+            k++;
+        }
+    }
     BigFix r;
     r.limbs = L;
     for (int k = 0; k <= L; k++) r.w[k] = p[k + L];
@@ -176,16 +168,8 @@ inline double bigfix_to_double(const BigFix &a)
         }
     if (top < 0) return 0.0;
     // take up to 128 bits from the top two limbs
-    // (a value of the top two places, as nearly all are, by exact constants)
-    const int e = top - a.limbs;
-    double hi, lo;
-    if (e >= -1 && top > 0) {
-        hi = (double)a.w[top] * (e == 0 ? 1.0 : 0x1p-64);
-        lo = (double)a.w[top - 1] * (e == 0 ? 0x1p-64 : 0x1p-128);
-    } else {
-        hi = std::ldexp((double)a.w[top], 64 * e);
-        lo = top > 0 ? std::ldexp((double)a.w[top - 1], 64 * (e - 1)) : 0.0;
-    }
+    double hi = std::ldexp((double)a.w[top], 64 * (top - a.limbs));
+    double lo = top > 0 ? std::ldexp((double)a.w[top - 1], 64 * (top - 1 - a.limbs)) : 0.0;
     double v = hi + lo;
     return a.neg ? -v : v;
 }
