@@ -61,6 +61,7 @@
 
 namespace chaos {
 int api_fail(int code, const char *fmt, ...);  // chaos_api.cu
+void api_prefault(void *p, size_t bytes);      // chaos_api.cu
 int api_orbit_create_d(double center_x, double center_y, uint32_t bits, uint32_t max_iterations,
                        chaos_orbit **out);  // chaos_perturb.cu
 int api_perturb_enqueue(const chaos_frame_desc *desc, const chaos_orbit *orbit, const chaos_frame_out *out,
@@ -1381,6 +1382,7 @@ int chaos_server_read(chaos_server *s, uint32_t session, uint32_t *host_rgba, un
     // the session's frames have finished (their launches ended), and none is
     // admitted while reading: plain copies
     cudaError_t e = cudaSuccess;
+    if (host_rgba) api_prefault(host_rgba, 4u * (size_t)w * h);
     if (host_rgba) e = cudaMemcpy2D(host_rgba, 4u * (size_t)w, rgba, rp, 4u * (size_t)w, h, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && pixel_iterations)
         e = cudaMemcpy(pixel_iterations, iters, sizeof(unsigned long long), cudaMemcpyDeviceToHost);
