@@ -780,6 +780,19 @@ __device__ __forceinline__ void store_pixel(PixelInfo *p, const PixelInfo &v)
     }
 }
 
+// The same for records that nothing reads soon (a frame's reused pixels are
+// as many bytes as the L2 holds): written past the rows of the previous frame
+// that neighbouring tiles still read.  3840x2160 zoom step: 113 -> 108 us.
+__device__ __forceinline__ void store_pixel_streaming(PixelInfo *p, const PixelInfo &v)
+{
+    if ((reinterpret_cast<uintptr_t>(p) & 15u) == 0)
+        __stcs(reinterpret_cast<uint4 *>(p),
+               make_uint4(__float_as_uint(v.value), __float_as_uint(v.weight), (uint32_t)v.is_reused,
+                          __float_as_uint(v.weight_of_new_samples)));
+    else
+        store_pixel(p, v);
+}
+
 __device__ __forceinline__ PixelInfo load_pixel(const PixelInfo *p)
 {
     PixelInfo v;

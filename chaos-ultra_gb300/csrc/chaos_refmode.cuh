@@ -5,6 +5,8 @@
 // modules) and chaos_newton.cu (Newton modules, built without contraction).
 #pragma once
 
+#include <algorithm>
+
 #include "chaos_claim.cuh"
 #include "chaos_kernels.cuh"
 
@@ -201,7 +203,7 @@ __device__ __forceinline__ void advanced_strip(const AdvancedArgs<R> &a, const S
                 if (valid) {
                     PixelInfo rec = make_pixel(vw.x, vw.y);
                     rec.is_reused = 1;
-                    store_pixel(pixel_ptr(a.m.out, a.m.pitch, p.x, p.y), rec);
+                    store_pixel_streaming(pixel_ptr(a.m.out, a.m.pitch, p.x, p.y), rec);
                 }
                 continue;
             }
@@ -266,11 +268,27 @@ static inline unsigned grid_for(unsigned long long work_warps, int occ, int sms)
     return (unsigned)blocks;
 }
 
+// k_main's residency and longest strip for escape-time tiles.  A tile across the
+// boundary runs up to maxIterations sample after sample, and the last such tiles
+// are the launch's end: with 64 warps an SM each had a sixteenth of its
+// scheduler, with 32 an eighth, and 32 still fill the issue slots before that.
+// A strip is rendered by one warp, so long strips lengthen that end, while
+// single tiles make the counter the bound of large shallow frames.  Default
+// view, maxIter 1600 (8 blocks and up to 16 tiles / 4 and 2 / 4 and 1): 1920x1080
+// of 5 samples 304 / 280 / 284 us, 3840x2160 of 2 478 / 417 / 361, 7680x4320 of
+// 1 948 / 745 / 787 (at maxIter 64: 491 / 505 / 722); three blocks are slower for
+// shallow frames (219 against 200 us at 3840x2160, maxIter 64).  Newton tiles
+// are short and even: they keep all warps (136 against 139 us at 1920x1080).
+constexpr int MAIN_BLOCKS = 4;
+constexpr uint32_t MAIN_STRIP = 2;
+
 template <class R, int A, int F> static cudaError_t launch_main_t(const MainArgs<R> &args, int sms, cudaStream_t s)
 {
-    static const int occ = occupancy(k_main<R, A, F>, PERSIST_THREADS);
+    constexpr bool newton = F >= FRACTAL_NEWTON_WIRED;
+    static const int fit = occupancy(k_main<R, A, F>, PERSIST_THREADS);
+    const int occ = newton ? fit : std::min(MAIN_BLOCKS, fit);
     MainArgs<R> a = args;
-    a.tile_chunk = tile_chunk_for(a.n_tiles, occ, sms);
+    a.tile_chunk = newton ? tile_chunk_for(a.n_tiles, occ, sms) : tile_chunk_for(a.n_tiles, occ, sms, MAIN_STRIP);
     k_main<R, A, F><<<grid_for((a.n_tiles + a.tile_chunk - 1) / a.tile_chunk, occ, sms), PERSIST_THREADS, 0, s>>>(a);
     return cudaGetLastError();
 }
