@@ -190,11 +190,10 @@ __device__ __forceinline__ void renormalise(D &dx, D &dy, D &dcx, D &dcy, int &e
     }
 }
 
-// Four blocks of 256 per SM for binary32 differences, three for binary64 (64 and
-// 80 registers): five and four measured 158.5 against 158.0 us at 1920x1080,
-// span 1e-200, 63.9 against 61.8 at 1280x720, 1e-25, and 826 against 817 in
-// binary64
-template <class D, int K, bool S> __global__ void __launch_bounds__(256, sizeof(D) == 4 ? 4 : 3) k_perturb(PerturbArgs<D> a)
+// Five blocks of 256 per SM for binary32 differences (48 registers: the
+// kernel is issue-bound and a sixth warp per scheduler hides more of the
+// orbit loads than extra registers save), four for binary64 (64 registers)
+template <class D, int K, bool S> __global__ void __launch_bounds__(256, sizeof(D) == 4 ? 5 : 4) k_perturb(PerturbArgs<D> a)
 {
     static_assert(!S || sizeof(D) == 4, "rescaling is for binary32 differences");
     using O = Op<D>;
