@@ -314,9 +314,16 @@ int api_fail(int code, const char *fmt, ...)
 // fill.  A caller's fresh buffer has no pages yet, and the copy engine took 27
 // ms to fault in the eight 1280x720 images that it copies in 1.3 ms otherwise;
 // from the CPU the same pages take about a tenth of that.  (The buffer's
-// contents are undefined until the copy anyway.)
+// contents are undefined until the copy anyway.)  Memory that CUDA knows (pinned,
+// managed, or a device address, which the copy refuses) is left alone.
 void api_prefault(void *p, size_t bytes)
 {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();  // not a CUDA error of the caller's
+        return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return;
     static const size_t page = [] {
         const long n = sysconf(_SC_PAGESIZE);
         return n > 0 ? (size_t)n : (size_t)4096;

@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(frame32_threads<MULTI>()) k_frame32(FrameArgs<
             tested = n < (uint32_t)LONG_STEPS && n + (uint32_t)ESCAPE_BLOCK <= rest;
         }
         if (tested) {
-            tested_steps<float, A>(x, y, cx, cy, i, min(i + (uint32_t)LONG_STEPS, a.max_iter), r2);
+            tested_steps<float, A>(x, y, cx, cy, i, a.max_iter - i > (uint32_t)LONG_STEPS ? i + LONG_STEPS : a.max_iter, r2);
             if (!(r2 < 4.f) || i == a.max_iter) return true;
             if (cw.check(x, y)) {
                 skipped += a.max_iter - i;
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(frame32_threads<MULTI>()) k_frame32(FrameArgs<
                 if (live) {
                     bool ended = start();
                     if (!ended) {
-                        const uint32_t end = min(i + (uint32_t)FRESH_STEPS, a.max_iter);
+                        const uint32_t end = a.max_iter - i > (uint32_t)FRESH_STEPS ? i + FRESH_STEPS : a.max_iter;
                         tested_steps<float, A>(x, y, cx, cy, i, end, r2);
                         ended = !(r2 < 4.f) || i == a.max_iter;
                     }
