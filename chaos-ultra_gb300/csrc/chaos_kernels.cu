@@ -845,13 +845,8 @@ template <int A, int F> static cudaError_t launch_frame64(const FrameArgs<double
 {
     static const int occ = occupancy(k_frame<A, F>, PERSIST_THREADS);
     unsigned long long warps = ((unsigned long long)a.n_pix + 31ull) / 32ull;
-    // frames of fewer warps than eight an SM spread over all SMs (each has its own
-    // binary64 pipe) in smaller blocks
-    const unsigned long long per_sm = (warps + (unsigned)sms - 1ull) / (unsigned)sms;
-    const unsigned threads = per_sm >= PERSIST_THREADS / 32 ? PERSIST_THREADS : 32u * (unsigned)per_sm;
-    const unsigned long long blocks = (warps + threads / 32u - 1ull) / (threads / 32u);
-    const unsigned grid = (unsigned)std::min(blocks, (unsigned long long)occ * (unsigned)sms);
-    k_frame<A, F><<<grid, threads, 0, s>>>(a);
+    const LaunchShape l = shape_for(warps, occ, sms);
+    k_frame<A, F><<<l.blocks, l.threads, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -272,7 +272,8 @@ static cudaError_t launch_serve_t(const ServeFrame<R> *frames, const uint32_t *b
                                   uint32_t n_jobs, uint32_t *counter, const ServeLaunchArgs &L, cudaStream_t s)
 {
     const int occ = serve_occupancy<R, A, F, ADV>();
-    k_serve<R, A, F, ADV><<<grid_for(n_jobs, occ, L.sms), PERSIST_THREADS, 0, s>>>(
+    const LaunchShape l = shape_for(n_jobs, occ, L.sms);
+    k_serve<R, A, F, ADV><<<l.blocks, l.threads, 0, s>>>(
         frames, begin, n_frames, counter, L.status, L.jobs_done, L.done_words, L.totals, L.budget_ns, L.palette,
         L.palette_len);
     return cudaGetLastError();
