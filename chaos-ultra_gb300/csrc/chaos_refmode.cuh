@@ -291,14 +291,18 @@ static inline LaunchShape shape_for(unsigned long long work_warps, int occ, int 
 // 1 948 / 745 / 787 (at maxIter 64: 491 / 505 / 722); three blocks are slower for
 // shallow frames (219 against 200 us at 3840x2160, maxIter 64).  Newton tiles
 // are short and even: they keep all warps (136 against 139 us at 1920x1080).
-constexpr int MAIN_BLOCKS = 4;
+// Binary64 tiles queue for one pipe, which four warps a scheduler fill: two
+// blocks (with 1 / 2 / 4: 500x300 of 2 samples 7.71 / 7.42 / 7.93 ms, 853x479 of 1
+// 14.29 / 13.91 / 14.00, 640x400 of 4 24.07 / 23.08 / 23.11).  Float-float ones are
+// binary32 work.
+template <class R, int A> constexpr int main_blocks() { return sizeof(R) == 8 && A != ARITH_FLOATFLOAT ? 2 : 4; }
 constexpr uint32_t MAIN_STRIP = 2;
 
 template <class R, int A, int F> static cudaError_t launch_main_t(const MainArgs<R> &args, int sms, cudaStream_t s)
 {
     constexpr bool newton = F >= FRACTAL_NEWTON_WIRED;
     static const int fit = occupancy(k_main<R, A, F>, PERSIST_THREADS);
-    const int occ = newton ? fit : std::min(MAIN_BLOCKS, fit);
+    const int occ = newton ? fit : std::min(main_blocks<R, A>(), fit);
     MainArgs<R> a = args;
     a.tile_chunk = newton ? tile_chunk_for(a.n_tiles, occ, sms) : tile_chunk_for(a.n_tiles, occ, sms, MAIN_STRIP);
     const LaunchShape l = shape_for((a.n_tiles + a.tile_chunk - 1) / a.tile_chunk, occ, sms);
