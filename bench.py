@@ -349,7 +349,7 @@ def run_ours(args):
             "peak_source": "measured in this run: chaos_measure_fma_peak (full-occupancy DFMA chains)",
             "ops_per_iteration": ops_per_iter, "fp64_pipe_ops_per_iteration": pipe_ops_per_iter,
             "fp64_pipe_frac": rate * pipe_ops_per_iter / (peak / 2),
-            "kernel": "k_frame<double,PARITY,mandelbrot>",
+            "kernel": "k_frame<PARITY,mandelbrot>",
             "note": "algorithmic ops = 6 per pixel-iteration (3 products, 2 adds, 1 fused add); one of them (x*x - y*y) runs "
                     "exactly rounded on the integer units, so frac can exceed 1; fp64_pipe_frac counts the 5 "
                     "FP64-pipe instructions per iteration"}
@@ -931,12 +931,12 @@ def run_c1(args):
     roof = {"bound": "fp32-pipe", "achieved": achieved / 1e12, "peak": peak / 2 / 1e12, "unit": "Top/s",
             "frac": achieved / (peak / 2), "traffic": None, "ops_per_iteration": ops,
             "peak_source": "measured in this run: chaos_measure_fma_peak (full-occupancy FFMA chains)",
-            "kernel": "k_frame<float,PARITY,mandelbrot,64>",
+            "kernel": "k_frame32<PARITY,mandelbrot,false>",
             "steps_executed_per_frame": executed, "pixel_iterations_per_frame": per_frame,
             "frac_of_steps_executed": executed / (ms / args.steps / 1e3) * ops / (peak / 2),
-            "note": "pixel-iterations count an interior sample as maxIter (the metric's unit); the kernel stops a "
-                    "sample whose rounded state repeats bit for bit (exact cycle detection), so it executes fewer "
-                    "steps: frac uses pixel-iterations, frac_of_steps_executed the steps the FP32 pipe ran"}
+            "note": "pixel-iterations count an interior sample as maxIter (the metric's unit); the kernel "
+                    "answers a sample inside the main cardioid or the period-2 disc without a step and stops one "
+                    "whose rounded state repeats bit for bit (exact cycle detection), so it executes fewer steps: frac uses pixel-iterations, frac_of_steps_executed the steps the FP32 pipe ran"}
 
     # CPU leg: the reference's computeFractal<float> over the whole frame, all host threads
     cpu = None

@@ -31,8 +31,8 @@
 // w' = P w + Q u.  The same composed map also stands in for 16 full steps of a
 // binary32 difference at e >= -126 or a plain one, while the difference stays
 // so far below the orbit over the block that the dropped d^2 term is below
-// binary32 rounding (a per-index exponent bound, lin_lim, set on the host from
-// |Z_j| and the partial products); 64-step maps go first where their bound
+// binary32 rounding (a per-index exponent bound, lin_lim, set by k_orbit_tables
+// from |Z_j| and the partial products); 64-step maps go first where their bound
 // allows.  Binary64 differences have their own 16- and 64-step maps and bounds
 // (binary64 rounding); where those do not apply, short linear steps run
 // while |d| and |dc| stay below 2^-120 and both components of Z above 2^-20:
@@ -467,7 +467,7 @@ template <class D, int K, bool S> __global__ void __launch_bounds__(256, sizeof(
                         const float ux = (float)dcx, uy = (float)dcy;
                         const float2 *Z2p = a.orbit2 + m;
                         if (n == B) {
-                            // the usual case: a whole block, its 16 steps composed on the host
+                            // the usual case: a whole block, its 16 steps composed by k_orbit_tables
                             // into w' = P w + Q u (one 16-byte load, eight operations)
                             const float4 pq = a.bla16[m];
                             const float nx =
@@ -800,9 +800,9 @@ struct OrbitTables {
 // (|w|, |u| <= 2^25 before it): 2 (|P|^2 + |Q|^2) <= 2^200.  A bound below -127
 // is stored as none.
 //
-// Bound: the binary64 pipe's latency, 15 operations a step for 64 steps
-// (about 35 us for orbits that fill less than the chip, whatever their
-// length; the least ratio is found by cross-multiplication, its one division
+// Bound: the binary64 pipe's latency, 15 operations a step for 64 steps (47 us
+// for 931 indices and both types; any orbit that fills less than the chip takes
+// as long.  The least ratio is found by cross-multiplication, its one division
 // at the end).  On the host, 931 indices took 0.2 to 0.4 ms on up to eight
 // threads for each type, and 156 bytes an index went to the device instead of
 // 24.  Blocks of 64 threads: an orbit of 1000 entries spreads over 32 SMs.
