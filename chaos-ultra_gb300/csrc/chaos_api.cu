@@ -24,6 +24,7 @@
 
 #include "../../include/chaos_gb300.h"
 #include "chaos_kernels.cuh"
+#include "chaos_slots.h"
 #include "chaos_trace.h"
 
 using namespace chaos;
@@ -56,11 +57,13 @@ int cuda_fail(cudaError_t e, const char *what)
         if (e_ != cudaSuccess) return cuda_fail(e_, what); \
     } while (0)
 
-// Per-device state: SM count and a ring of work counters.  Each persistent
-// launch takes the next slot, so launches in flight on different streams use
-// different counters (up to kCounterSlots of them at once).  A slot is a work
-// counter and its companion (zero between launches: the kernels leave them so,
-// see leave_counter) and a status word.
+// Per-device state: SM count and the work counters of the persistent launches.
+// A slot is a counter, a status word and (tracked slots) a count of ended blocks.
+//   0 .. kCounterSlots - 1                 tracked: a slot goes out again when its
+//       launch has ended (chaos_slots.h), and the kernels leave its words at zero
+//   kCounterSlots .. 2 kCounterSlots - 1   zeroed by a memset on the launch's
+//       stream and taken in turn: launches recorded in a graph, whose replays the
+//       host does not see, and those beside kCounterSlots others in flight
 constexpr int kMaxDevices = 64;
 constexpr uint32_t kCounterSlots = 4096;
 
@@ -68,8 +71,10 @@ struct DeviceState {
     std::once_flag once;
     cudaError_t init_error = cudaSuccess;
     int sms = 0;
-    uint32_t *counters = nullptr;
-    std::atomic<uint32_t> next{0};
+    uint32_t *counters = nullptr;  // 2 kCounterSlots each of counters and status words, then the ended blocks
+    uint32_t *busy = nullptr;      // the tracked slots' words as the device sees them
+    SlotRing ring;
+    std::atomic<uint32_t> next_zeroed{0};
 };
 DeviceState g_devices[kMaxDevices];
 
@@ -80,11 +85,19 @@ int device_state(DeviceState **out)
     if (dev < 0 || dev >= kMaxDevices) return fail(CHAOS_ERR_UNSUPPORTED, "device %d out of range", dev);
     DeviceState &d = g_devices[dev];
     std::call_once(d.once, [&]() {
+        constexpr size_t words = 5 * kCounterSlots;
         cudaError_t e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess) e = cudaMalloc(&d.counters, 3 * kCounterSlots * sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaMalloc(&d.counters, words * sizeof(uint32_t));
         // (on the legacy stream, and waited for: the first launch may be on any other)
-        if (e == cudaSuccess) e = cudaMemset(d.counters, 0, 3 * kCounterSlots * sizeof(uint32_t));
+        if (e == cudaSuccess) e = cudaMemset(d.counters, 0, words * sizeof(uint32_t));
         if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+        uint32_t *busy = nullptr;
+        if (e == cudaSuccess) e = cudaHostAlloc(&busy, kCounterSlots * sizeof(uint32_t), cudaHostAllocMapped);
+        if (e == cudaSuccess) {
+            std::memset(busy, 0, kCounterSlots * sizeof(uint32_t));
+            d.ring.init(busy, kCounterSlots);
+            e = cudaHostGetDevicePointer(&d.busy, busy, 0);
+        }
         d.init_error = e;
     });
     if (d.init_error != cudaSuccess) return cuda_fail(d.init_error, "device set-up");
@@ -92,18 +105,26 @@ int device_state(DeviceState **out)
     return CHAOS_OK;
 }
 
-void take_counter(DeviceState *d, uint32_t **counter, uint32_t **done)
+int take_counter(DeviceState *d, cudaStream_t s, WorkCounter *work)
 {
-    uint32_t slot = d->next.fetch_add(1, std::memory_order_relaxed) % kCounterSlots;
-    *counter = d->counters + slot;
-    *done = d->counters + 2 * kCounterSlots + slot;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CHAOS_CUDA(cudaStreamIsCapturing(s, &capture), "cudaStreamIsCapturing");
+    const uint32_t slot = capture == cudaStreamCaptureStatusNone ? d->ring.take() : SlotRing::NONE;
+    if (slot != SlotRing::NONE) {
+        *work = WorkCounter{d->counters + slot, d->counters + 4 * kCounterSlots + slot, d->busy + slot};
+        return CHAOS_OK;
+    }
+    const uint32_t k = d->next_zeroed.fetch_add(1, std::memory_order_relaxed) % kCounterSlots;
+    *work = WorkCounter{d->counters + kCounterSlots + k, nullptr, nullptr};
+    CHAOS_CUDA(cudaMemsetAsync(work->next, 0, sizeof(uint32_t), s), "cudaMemsetAsync(work counter)");
+    return CHAOS_OK;
 }
 
-// The status word that goes with a counter slot (a launch with a time limit
+// The status word that goes with a counter (a launch with a time limit
 // and no status word of the caller's), zeroed on the stream.
-int take_status(const DeviceState *d, const uint32_t *counter, cudaStream_t s, uint32_t **status)
+int take_status(const DeviceState *d, const WorkCounter &work, cudaStream_t s, uint32_t **status)
 {
-    *status = d->counters + kCounterSlots + (counter - d->counters);
+    *status = d->counters + 2 * kCounterSlots + (work.next - d->counters);
     CHAOS_CUDA(cudaMemsetAsync(*status, 0, sizeof(uint32_t), s), "cudaMemsetAsync(status word)");
     return CHAOS_OK;
 }
@@ -333,22 +354,21 @@ void api_prefault(void *p, size_t bytes)
     if (bytes) c[bytes - 1] = 0;
 }
 
-int api_device_counter(uint32_t **counter, uint32_t **done, int *sms)
+int api_device_counter(cudaStream_t s, WorkCounter *work, int *sms)
 {
     DeviceState *d;
     int rc = device_state(&d);
     if (rc) return rc;
     *sms = d->sms;
-    take_counter(d, counter, done);
-    return CHAOS_OK;
+    return take_counter(d, s, work);
 }
 
-int api_device_status(const uint32_t *counter, cudaStream_t s, uint32_t **status)
+int api_device_status(const WorkCounter &work, cudaStream_t s, uint32_t **status)
 {
     DeviceState *d;
     int rc = device_state(&d);
     if (rc) return rc;
-    return take_status(d, counter, s, status);
+    return take_status(d, work, s, status);
 }
 
 bool api_budget(double seconds, unsigned long long *ns) { return budget_of(seconds, ns); }
@@ -552,7 +572,7 @@ static int render_main(chaos_module *m, chaos_pixel_info *out, long pitch, uint3
     a.newton = m->newton;
     a.tiles_x = (w + 7u) / 8u;
     a.n_tiles = a.tiles_x * ((h + 3u) / 4u);
-    take_counter(d, &a.counter, &a.done);
+    if ((rc = take_counter(d, s, &a.work))) return rc;
     return finish(launch_main<R>(a, arith_of(arith), m->fractal, d->sms, s), s, sync);
 }
 
@@ -594,7 +614,7 @@ static int render_advanced(chaos_module *m, chaos_pixel_info *out, long pitch, u
     a.in = in;
     a.in_pitch = in_pitch;
     a.focus = UInt2{fx, fy};
-    take_counter(d, &a.m.counter, &a.m.done);
+    if ((rc = take_counter(d, s, &a.m.work))) return rc;
     return finish(launch_advanced<R>(a, arith_of(arith), m->fractal, d->sms, s), s, sync);
 }
 
@@ -746,13 +766,12 @@ static int frame_impl(const chaos_frame_desc *dsc, const chaos_frame_out *o, cud
     a.total = o->total_iterations;
     a.skipped = o->cycle_skipped;
     budget_of(dsc->time_limit_s, &a.budget_ns);
-    take_counter(d, &a.counter, &a.done);
     a.status = o->status;
-    if (a.budget_ns && !a.status) {
-        if (!sync && !status_used)
-            return fail(CHAOS_ERR_INVALID_ARGUMENT, "a time limit on an unsynchronised frame needs out->status");
-        if ((rc = take_status(d, a.counter, s, &a.status))) return rc;
-    }
+    const bool own_status = a.budget_ns && !a.status;
+    if (own_status && !sync && !status_used)
+        return fail(CHAOS_ERR_INVALID_ARGUMENT, "a time limit on an unsynchronised frame needs out->status");
+    if ((rc = take_counter(d, s, &a.work))) return rc;
+    if (own_status && (rc = take_status(d, a.work, s, &a.status))) return rc;
     if (status_used) *status_used = a.budget_ns ? a.status : nullptr;
     if ((rc = finish(launch_frame<R>(a, arith_of(dsc->arith), (int)dsc->fractal, d->sms, s), s, sync))) return rc;
     return sync && a.budget_ns ? read_status(a.status, s, dsc->time_limit_s) : CHAOS_OK;

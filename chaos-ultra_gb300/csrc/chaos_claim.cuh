@@ -16,19 +16,31 @@
 
 namespace chaos {
 
+// A launch's work counter (`next`; zero when the launch starts) and its slot's
+// other words, null where the caller or a memset before the launch zeroes the
+// counter: the number of blocks that have ended (zero between launches) and the
+// host's word that says the slot is taken (chaos_slots.h).
+struct WorkCounter {
+    uint32_t *next, *done, *busy;
+};
+
 // The end of a persistent kernel: the launch's last warp leaves the work counter
 // at zero for the launch that takes it next (a memset before every launch cost
-// a small frame as much as its kernel).  Each warp's lane 0 calls it after the
-// warp's last claim.  retired: shared, zero from before the block's first
-// barrier; done: the counter's companion word, zero between launches, or null
-// where the caller zeroes the counter.
-__device__ __forceinline__ void leave_counter(uint32_t *counter, uint32_t *done, uint32_t *retired)
+// a small frame as much as its kernel) and gives the slot back.  Each warp's
+// lane 0 calls it after the warp's last claim.  retired: shared, zero from before
+// the block's first barrier.  No claim is still on its way when the words go back
+// to zero: a warp gets here by the result of its last one.  (The host's word
+// follows them at system scope; 20.2 -> 20.5 us for a 256x144 frame.  A fence in
+// every block waited for the block's pixels: 166 -> 168 us at 1920x1080.)
+__device__ __forceinline__ void leave_counter(const WorkCounter &w, uint32_t *retired)
 {
-    if (!done) return;
+    if (!w.done) return;
     if (atomicAdd(retired, 1u) + 1u != (blockDim.x >> 5)) return;
-    if (atomicAdd(done, 1u) + 1u != gridDim.x) return;
-    *counter = 0u;
-    *done = 0u;
+    if (atomicAdd(w.done, 1u) + 1u != gridDim.x) return;
+    *w.next = 0u;
+    *w.done = 0u;
+    __threadfence_system();
+    *(volatile uint32_t *)w.busy = 0u;
 }
 
 // Pieces of `size` items; the first of every block goes out without a claim

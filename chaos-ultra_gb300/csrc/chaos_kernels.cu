@@ -160,7 +160,7 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
                     first = false;
                 } else {
                     const uint32_t leader = __ffs(need_mask) - 1u;
-                    if (lane == leader) base = 32u * n_warps + atomicAdd(a.counter, (uint32_t)__popc(need_mask));
+                    if (lane == leader) base = 32u * n_warps + atomicAdd(a.work.next, (uint32_t)__popc(need_mask));
                     base = __shfl_sync(FULL, base, leader);
                 }
                 if (need) {
@@ -362,7 +362,7 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
         for (int o = 16; o > 0; o >>= 1) skipped += __shfl_down_sync(FULL, skipped, o);
         if (lane == 0 && skipped) atomicAdd(a.skipped, skipped);
     }
-    if (lane == 0) leave_counter(a.counter, a.done, &s_retired);
+    if (lane == 0) leave_counter(a.work, &s_retired);
 }
 
 // ---------------------------------------------------------------------------
@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(frame32_threads<MULTI>()) k_frame32(FrameArgs<
             if (round < fixed_rounds) {
                 base = 32u * (round++ * n_warps + warp);
             } else {
-                if (lane == 0) base = claim_base + atomicAdd(a.counter, 32u);
+                if (lane == 0) base = claim_base + atomicAdd(a.work.next, 32u);
                 base = __shfl_sync(FULL, base, 0);
             }
             if (base >= a.n_pix) {
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(frame32_threads<MULTI>()) k_frame32(FrameArgs<
         for (int o = 16; o > 0; o >>= 1) skipped += __shfl_down_sync(FULL, skipped, o);
         if (lane == 0 && skipped) atomicAdd(a.skipped, skipped);
     }
-    if (lane == 0) leave_counter(a.counter, a.done, &s_retired);
+    if (lane == 0) leave_counter(a.work, &s_retired);
 }
 
 // ---------------------------------------------------------------------------

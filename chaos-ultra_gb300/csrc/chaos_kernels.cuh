@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "chaos_claim.cuh"
 #include "chaos_device.cuh"
 
 namespace chaos {
@@ -36,7 +37,7 @@ template <class R> struct MainArgs {
     uint32_t flags;
     double jcx, jcy;
     uint32_t tiles_x, n_tiles;
-    uint32_t *counter, *done;   // see leave_counter
+    WorkCounter work;
     unsigned long long *total;  // optional: pixel-iterations of the samples taken
     NewtonParams newton;        // Newton modules only
     uint32_t tile_chunk;        // tiles per claim (set by the launcher)
@@ -64,7 +65,7 @@ template <class R> struct FrameArgs {
     uint32_t palette_len;
     uint32_t interior_rgba;
     unsigned long long *total;
-    uint32_t *counter, *done;     // see leave_counter
+    WorkCounter work;
     unsigned long long *skipped;  // optional: iterations of interior samples proven by a repeated state, not run
     unsigned long long budget_ns; // 0, or the run time after which warps stop (RUN_STATUS_TIMEOUT into *status)
     uint32_t *status;

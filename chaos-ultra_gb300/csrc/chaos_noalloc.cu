@@ -100,7 +100,7 @@ cudaError_t launch(const chaos_frame_desc *d, unsigned char *base, uint32_t pale
     a.half_h = (R)(0.5 * d->height);
     a.jcx = (R)d->julia_cx;
     a.jcy = (R)d->julia_cy;
-    a.counter = reinterpret_cast<uint32_t *>(base);
+    a.work.next = reinterpret_cast<uint32_t *>(base);
     a.total = reinterpret_cast<unsigned long long *>(base + 8);
     a.palette = reinterpret_cast<const uint32_t *>(base + kHeaderBytes);
     a.palette_len = palette_len;

@@ -57,8 +57,8 @@
 namespace chaos {
 
 int api_fail(int code, const char *fmt, ...);  // chaos_api.cu
-int api_device_counter(uint32_t **counter, uint32_t **done, int *sms);
-int api_device_status(const uint32_t *counter, cudaStream_t s, uint32_t **status);
+int api_device_counter(cudaStream_t s, WorkCounter *work, int *sms);
+int api_device_status(const WorkCounter &work, cudaStream_t s, uint32_t **status);
 bool api_budget(double seconds, unsigned long long *ns);
 int api_read_status(const uint32_t *status, cudaStream_t s, double seconds);
 
@@ -99,7 +99,7 @@ template <class D> struct PerturbArgs {
     uint32_t interior_rgba;
     unsigned long long *total;
     unsigned long long *rebases;
-    uint32_t *counter, *done;      // see leave_counter
+    WorkCounter work;
     unsigned long long budget_ns;  // 0, or the run time after which warps stop (RUN_STATUS_TIMEOUT into *status)
     uint32_t *status;
     // binary32 set-up of rescaled samples at pixel centres (dc_fast): with
@@ -229,7 +229,7 @@ template <class D, int K, bool S> __global__ void __launch_bounds__(256, sizeof(
         if (need_mask) {
             uint32_t leader = __ffs(need_mask) - 1u;
             uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(a.counter, (uint32_t)__popc(need_mask));
+            if (lane == leader) base = atomicAdd(a.work.next, (uint32_t)__popc(need_mask));
             base = __shfl_sync(FULLM, base, leader);
             if (need) {
                 pix = base + (uint32_t)__popc(need_mask & lt_mask);
@@ -682,7 +682,7 @@ template <class D, int K, bool S> __global__ void __launch_bounds__(256, sizeof(
     if (lane == 0) {
         if (a.total && iters) atomicAdd(a.total, iters);
         if (a.rebases && rebases) atomicAdd(a.rebases, rebases);
-        leave_counter(a.counter, a.done, &s_retired);
+        leave_counter(a.work, &s_retired);
     }
 }
 
@@ -1092,20 +1092,21 @@ static int perturb_impl(const chaos_frame_desc *d, const chaos_orbit *orb, const
     a.status = o->status;
     if (!api_budget(d->time_limit_s, &a.budget_ns))
         return api_fail(CHAOS_ERR_INVALID_ARGUMENT, "time_limit_s must be >= 0");
+    const bool own_status = a.budget_ns && !a.status;
+    if (own_status && (!sync || counter))
+        return api_fail(CHAOS_ERR_INVALID_ARGUMENT, "a time limit on an unsynchronised frame needs out->status");
     int sms = 0;
     if (counter) {
-        a.counter = counter;
+        a.work.next = counter;
         int dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     } else {
-        int rc = api_device_counter(&a.counter, &a.done, &sms);
+        int rc = api_device_counter(s, &a.work, &sms);
         if (rc) return rc;
     }
-    if (a.budget_ns && !a.status) {
-        if (!sync || counter)
-            return api_fail(CHAOS_ERR_INVALID_ARGUMENT, "a time limit on an unsynchronised frame needs out->status");
-        int rc = api_device_status(a.counter, s, &a.status);
+    if (own_status) {
+        int rc = api_device_status(a.work, s, &a.status);
         if (rc) return rc;
     }
     // binary32 differences are rescaled below pixel 1e-30 (2^-100)

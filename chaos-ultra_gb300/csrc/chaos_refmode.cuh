@@ -125,11 +125,11 @@ template <class R, int A, int F> __global__ void __launch_bounds__(PERSIST_THREA
     SampleGeometry<R> g = make_geometry(a.image, a.size, a.max_iter, a.jcx, a.jcy);
     g.newton = a.newton;
     unsigned long long iters = 0;
-    for_each_tile(a.counter, a.n_tiles, a.tiles_x, a.tile_chunk, lane, [&](uint32_t x0, uint32_t y0) {
+    for_each_tile(a.work.next, a.n_tiles, a.tiles_x, a.tile_chunk, lane, [&](uint32_t x0, uint32_t y0) {
         render_main_tile<R, A, F>(g, a.out, a.pitch, a.size, x0, y0, lane, a.max_ss, a.flags, iters);
     });
     add_total(a.total, iters, lane);
-    if (lane == 0) leave_counter(a.counter, a.done, &s_retired);
+    if (lane == 0) leave_counter(a.work, &s_retired);
 }
 
 constexpr uint32_t PIECE_TILES = 4 * PERSIST_THREADS / 32;  // a group of four for each warp
@@ -237,11 +237,11 @@ __global__ void __launch_bounds__(PERSIST_THREADS) k_advanced(AdvancedArgs<R> a)
     auto each = [&](auto strip) {
         if constexpr (PIECES) {
             __shared__ ClaimShared s_claims;
-            Claims claims(s_claims, a.m.counter, ClaimPlan{a.m.n_tiles, PIECE_TILES});
+            Claims claims(s_claims, a.m.work.next, ClaimPlan{a.m.n_tiles, PIECE_TILES});
             __syncthreads();
             for_each_claim(claims, 4u, strip);
         } else {
-            for_each_strip(a.m.counter, a.m.n_tiles, a.m.tile_chunk, lane, strip);
+            for_each_strip(a.m.work.next, a.m.n_tiles, a.m.tile_chunk, lane, strip);
         }
     };
     if (PIECES || al8)
@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS) k_advanced(AdvancedArgs<R> a)
     else
         each([&](uint32_t t0, uint32_t t1) { advanced_strip<R, A, F, false>(a, g, lane, stage, t0, t1, iters); });
     add_total(a.m.total, iters, lane);
-    if (lane == 0) leave_counter(a.m.counter, a.m.done, &s_retired);
+    if (lane == 0) leave_counter(a.m.work, &s_retired);
 }
 
 template <class KernelPtr> static int occupancy(KernelPtr k, int threads)
