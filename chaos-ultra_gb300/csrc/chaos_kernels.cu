@@ -176,7 +176,8 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
                 if (lane == 0) *(volatile uint32_t *)&s_drain = 1;
                 drain = true;
             } else {
-                drain = *(volatile uint32_t *)&s_drain != 0;
+                // (the lanes' reads may straddle the store; the warp decides as one)
+                drain = __any_sync(FULL, *(volatile uint32_t *)&s_drain != 0);
             }
             on = !need && pix < a.n_pix;
             rounds = 0;
