@@ -89,6 +89,9 @@ template <class R> __device__ __forceinline__ uint32_t newton_root(thrust::compl
     return 0;
 }
 
+// Whether four steps from step i end before step `end` (i <= end; i + 4 may wrap)
+__host__ __device__ constexpr bool newton_group(uint32_t i, uint32_t end) { return end - i > 4u; }
+
 // computeFractal of the three modules, as an unsigned value (the float the
 // reference returns is an integer): the root index (wired, generic) or the
 // iteration count (iterations).
@@ -126,7 +129,7 @@ template <class R, int F> __device__ uint32_t newton_compute(uint32_t max_iterat
     uint32_t check = 10;
     while (i < max_iterations) {
         const uint32_t end = min(check, max_iterations);
-        for (; i + 4u < end; i += 4u) {
+        for (; newton_group(i, end); i += 4u) {
             if (i > 8u) {
                 const thrust::complex<R> before = x;
                 x = step(x);
