@@ -17,12 +17,12 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <unistd.h>
 #include <mutex>
 #include <string>
 #include <vector>
 
 #include "../../include/chaos_gb300.h"
+#include "chaos_hostpages.h"
 #include "chaos_kernels.cuh"
 #include "chaos_slots.h"
 #include "chaos_trace.h"
@@ -331,12 +331,12 @@ int api_fail(int code, const char *fmt, ...)
     return code;
 }
 
-// Touches every page of a host buffer that a device-to-host copy is about to
+// Brings in the pages of a host buffer that a device-to-host copy is about to
 // fill.  A caller's fresh buffer has no pages yet, and the copy engine took 27
 // ms to fault in the eight 1280x720 images that it copies in 1.3 ms otherwise;
-// from the CPU the same pages take about a tenth of that.  (The buffer's
-// contents are undefined until the copy anyway.)  Memory that CUDA knows (pinned,
-// managed, or a device address, which the copy refuses) is left alone.
+// from the CPU the same pages take about a tenth of that.  Memory that CUDA
+// knows (pinned, managed, or a device address, which the copy refuses) is left
+// alone.
 void api_prefault(void *p, size_t bytes)
 {
     cudaPointerAttributes at{};
@@ -344,14 +344,7 @@ void api_prefault(void *p, size_t bytes)
         cudaGetLastError();  // not a CUDA error of the caller's
         return;
     }
-    if (at.type != cudaMemoryTypeUnregistered) return;
-    static const size_t page = [] {
-        const long n = sysconf(_SC_PAGESIZE);
-        return n > 0 ? (size_t)n : (size_t)4096;
-    }();
-    volatile char *c = static_cast<volatile char *>(p);
-    for (size_t k = 0; k < bytes; k += page) c[k] = 0;
-    if (bytes) c[bytes - 1] = 0;
+    if (at.type == cudaMemoryTypeUnregistered) populate_pages(p, bytes);
 }
 
 int api_device_counter(cudaStream_t s, WorkCounter *work, int *sms)
