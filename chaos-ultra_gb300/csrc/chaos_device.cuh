@@ -63,7 +63,8 @@ struct NewtonParams {
 
 // Newton-method value of a start point (chaos_newton.cuh; only the
 // translation units that render Newton fractals include its definition).
-template <class R, int F> __device__ uint32_t newton_compute(uint32_t max_iterations, R zx, R zy, const NewtonParams &p);
+template <class R, int F, bool AS_WRITTEN>
+__device__ uint32_t newton_compute(uint32_t max_iterations, R zx, R zy, const NewtonParams &p);
 
 // kernel flag bits, gen.cu:157-161 (bit 1 is the Java-side "visualise" flag)
 constexpr uint32_t FLAG_ADAPTIVE_SS = 1u << 0;
@@ -633,7 +634,7 @@ template <class R> struct SampleGeometry {
 template <class R, int A, int F> __device__ __forceinline__ uint32_t compute_fractal_g(const SampleGeometry<R> &g, R cx, R cy)
 {
     if constexpr (F >= FRACTAL_NEWTON_WIRED)
-        return newton_compute<R, F>(g.max_iter, cx, cy, g.newton);
+        return newton_compute<R, F, A == ARITH_CONTRACTED>(g.max_iter, cx, cy, g.newton);
     else
         return compute_fractal<R, A, F>(g.max_iter, cx, cy, g.jcx, g.jcy);
 }

@@ -19,7 +19,7 @@ __global__ void k_under_sampled_newton(void *out, long pitch, uint32_t w, uint32
     float ph = __fdiv_rn(__fsub_rn(r.rty, r.lby), (float)h);
     float cx = __fadd_rn(r.lbx, __fmul_rn((float)ix, pw));
     float cy = __fsub_rn(r.rty, __fmul_rn((float)iy, ph));
-    uint32_t e = newton_compute<float, F>(max_iter, cx, cy, p);
+    uint32_t e = newton_compute<float, F, false>(max_iter, cx, cy, p);
     store_pixel(pixel_ptr(out, pitch, ix, iy), make_pixel((float)e, __fdiv_rn(1.f, (float)level)));
 }
 

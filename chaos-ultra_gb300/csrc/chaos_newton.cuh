@@ -95,16 +95,47 @@ __host__ __device__ constexpr bool newton_group(uint32_t i, uint32_t end) { retu
 // computeFractal of the three modules, as an unsigned value (the float the
 // reference returns is an integer): the root index (wired, generic) or the
 // iteration count (iterations).
-// A state that a step leaves as it was, or that has become NaN (which stays
+//
+// AS_WRITTEN: the reference's loops around its step, for code built with nvcc's
+// contraction.  There the values are those of the products that nvcc fuses, and
+// it fuses within a basic block: a choice between two forms of the step, or
+// copies of it, moved some of them (640x360 pixels of the module's own
+// polynomial in binary32 came out otherwise).
+//
+// Otherwise a state that a step leaves as it was, or that has become NaN (which stays
 // so), is the state at every later test: the answer is the test's on it,
 // however many steps remain (looked at every fourth step).  Most start points settle bit for bit a few steps
 // after they come near a root, well before the test of step 30 where the one
 // of step 10 came too early.
 // (declared __forceinline__ in chaos_device.cuh; the attribute is not repeated here)
-template <class R, int F> __device__ uint32_t newton_compute(uint32_t max_iterations, R zx, R zy, const NewtonParams &p)
+template <class R, int F, bool AS_WRITTEN>
+__device__ uint32_t newton_compute(uint32_t max_iterations, R zx, R zy, const NewtonParams &p)
 {
     thrust::complex<R> x(zx, zy);
     const double *roots = F == FRACTAL_NEWTON_WIRED ? kWiredRoots : p.roots;
+    if constexpr (AS_WRITTEN) {
+        uint32_t i = 0;
+        if (F == FRACTAL_NEWTON_ITERATIONS) {  // newton_iterations.cu:54-67
+            while (i < max_iterations) {
+                x = newton_step_generic<R>(x, p.coefficients);
+                ++i;
+                if (newton_root<R>(x, roots) != 0) return i;
+            }
+            return i;
+        }
+        // newton_wired.cu:45-64, newton_generic.cu:53-72
+        uint32_t check = 10;
+        while (i < max_iterations) {
+            x = F == FRACTAL_NEWTON_WIRED ? newton_step_wired<R>(x) : newton_step_generic<R>(x, p.coefficients);
+            ++i;
+            if (i == check) {
+                uint32_t root = newton_root<R>(x, roots);
+                if (root != 0) return root;
+                check += max_iterations / 10;
+            }
+        }
+        return newton_root<R>(x, roots);
+    }
     const bool binomial = F != FRACTAL_NEWTON_WIRED && newton_binomial(p.coefficients, sizeof(R) == 4);
     const R c0 = (R)p.coefficients[0];
     auto step = [&](thrust::complex<R> z) {
