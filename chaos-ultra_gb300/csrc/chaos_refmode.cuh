@@ -280,23 +280,31 @@ static inline LaunchShape shape_for(unsigned long long work_warps, int occ, int 
     return {(unsigned)std::max(1ull, blocks), 32u * warps};
 }
 
-// k_main's residency and longest strip for escape-time tiles.  A tile across the
-// boundary runs up to maxIterations sample after sample, and the last such tiles
-// are the launch's end: with 64 warps an SM each had a sixteenth of its
-// scheduler, with 32 an eighth, and 32 still fill the issue slots before that.
-// A strip is rendered by one warp, so long strips lengthen that end, while
-// single tiles make the counter the bound of large shallow frames.  Default
-// view, maxIter 1600 (8 blocks and up to 16 tiles / 4 and 2 / 4 and 1): 1920x1080
-// of 5 samples 304 / 280 / 284 us, 3840x2160 of 2 478 / 417 / 361, 7680x4320 of
-// 1 948 / 745 / 787 (at maxIter 64: 491 / 505 / 722); three blocks are slower for
-// shallow frames (219 against 200 us at 3840x2160, maxIter 64).  Newton tiles
+// k_main's residency for escape-time tiles.  A tile across the boundary runs up
+// to maxIterations sample after sample, and the last such tiles are the launch's
+// end: with 64 warps an SM each had a sixteenth of its scheduler, with 32 an
+// eighth, and 32 still fill the issue slots before that (three blocks are slower
+// for shallow frames: 219 against 200 us at 3840x2160, maxIter 64).  Newton tiles
 // are short and even: they keep all warps (136 against 139 us at 1920x1080).
 // Binary64 tiles queue for one pipe, which four warps a scheduler fill: two
 // blocks (with 1 / 2 / 4: 500x300 of 2 samples 7.71 / 7.42 / 7.93 ms, 853x479 of 1
 // 14.29 / 13.91 / 14.00, 640x400 of 4 24.07 / 23.08 / 23.11).  Float-float ones are
 // binary32 work.
 template <class R, int A> constexpr int main_blocks() { return sizeof(R) == 8 && A != ARITH_FLOATFLOAT ? 2 : 4; }
-constexpr uint32_t MAIN_STRIP = 2;
+
+// And their longest strip.  One warp renders a strip, so its worst case, every
+// step of every sample, is held to a few tiles' share of what the frame gives a
+// warp; single tiles would make the counter the bound of large shallow frames.
+// Default view, us with strips of up to 2 / 4 / 8: 7680x4320, maxIter 16
+// 433 / 407 / 395, 64 509 / 489 / 485, 256 578 / 565 / 571, 1600 832 / 858 / 925
+// (all points outside, any limit: 388 / 357 / 344); 3840x2160, 16 128 / 121 / 119,
+// 64 147 / 146 / 148, 1600 279 / 312 / 346.
+static inline uint32_t main_strip(uint32_t n_tiles, int occ, int sms, uint32_t max_iter, float max_ss)
+{
+    const double tiles = (double)n_tiles / ((double)occ * sms * (PERSIST_THREADS / 32));  // a warp's
+    const double worst = std::max(1.0, (double)max_iter * std::max(1.0, (double)max_ss));
+    return (uint32_t)std::min(8.0, std::max(tiles >= 128.0 ? 4.0 : 2.0, 5.0 * tiles / worst));
+}
 
 template <class R, int A, int F> static cudaError_t launch_main_t(const MainArgs<R> &args, int sms, cudaStream_t s)
 {
@@ -304,7 +312,8 @@ template <class R, int A, int F> static cudaError_t launch_main_t(const MainArgs
     static const int fit = occupancy(k_main<R, A, F>, PERSIST_THREADS);
     const int occ = newton ? fit : std::min(main_blocks<R, A>(), fit);
     MainArgs<R> a = args;
-    a.tile_chunk = newton ? tile_chunk_for(a.n_tiles, occ, sms) : tile_chunk_for(a.n_tiles, occ, sms, MAIN_STRIP);
+    a.tile_chunk = newton ? tile_chunk_for(a.n_tiles, occ, sms)
+                          : tile_chunk_for(a.n_tiles, occ, sms, main_strip(a.n_tiles, occ, sms, a.max_iter, a.max_ss));
     const LaunchShape l = shape_for((a.n_tiles + a.tile_chunk - 1) / a.tile_chunk, occ, sms);
     k_main<R, A, F><<<l.blocks, l.threads, 0, s>>>(a);
     return cudaGetLastError();
