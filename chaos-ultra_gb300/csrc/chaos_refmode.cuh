@@ -24,15 +24,17 @@ __device__ __forceinline__ void add_total(unsigned long long *total, unsigned lo
     if (lane == 0 && iters) atomicAdd(total, iters);
 }
 
-// Tiles are claimed in strips of consecutive tiles, the next claim issued
-// before the current strip is rendered.  With one counter for the whole
-// frame, a claim per tile made the counter the bottleneck of large
+// Tiles are claimed in strips of consecutive tiles.  With one counter for the
+// whole frame, a claim per tile made the counter the bottleneck of large
 // reuse-dominated frames, whose tiles take a few loads each.  Claims are
 // guided: a quarter of an even share of the tiles left after the warp's
 // previous strip, between 1 and `max_chunk`, so long strips early keep the
-// counter quiet and short ones late keep the end of the frame balanced;
-// single tiles are claimed when needed (the finest balance, small frames).
-template <class Body>
+// counter quiet and short ones late keep the end of the frame balanced.
+// AHEAD (short, even tiles): a strip of several tiles is claimed before the one
+// before it is rendered.  Where a tile may run for long, the strip that its warp
+// holds already would wait as long, so strips are claimed when needed
+// (1801x1769, maxIter 1600, 5 samples, strips of two: 413 us ahead, 348).
+template <bool AHEAD, class Body>
 __device__ __forceinline__ void for_each_strip(uint32_t *counter, uint32_t n_tiles, uint32_t max_chunk, uint32_t lane,
                                                Body body)
 {
@@ -46,9 +48,10 @@ __device__ __forceinline__ void for_each_strip(uint32_t *counter, uint32_t n_til
     uint32_t t0 = __shfl_sync(FULL, claim, 0);
     while (t0 < n_tiles) {
         const uint32_t t1 = min(t0 + size, n_tiles), next = size_after(t1);
-        if (size > 1u && lane == 0) claim = atomicAdd(counter, next);
+        const bool ahead = AHEAD && size > 1u;
+        if (ahead && lane == 0) claim = atomicAdd(counter, next);
         body(t0, t1);
-        if (size == 1u && lane == 0) claim = atomicAdd(counter, next);
+        if (!ahead && lane == 0) claim = atomicAdd(counter, next);
         t0 = __shfl_sync(FULL, claim, 0);
         size = next;
     }
@@ -95,11 +98,11 @@ struct TileCursor {
 };
 
 // body(x0, y0) for every tile claimed, (x0, y0) its top-left pixel
-template <class Body>
+template <bool AHEAD, class Body>
 __device__ __forceinline__ void for_each_tile(uint32_t *counter, uint32_t n_tiles, uint32_t tiles_x, uint32_t chunk,
                                               uint32_t lane, Body body)
 {
-    for_each_strip(counter, n_tiles, chunk, lane, [&](uint32_t t0, uint32_t t1) {
+    for_each_strip<AHEAD>(counter, n_tiles, chunk, lane, [&](uint32_t t0, uint32_t t1) {
         TileCursor c(t0, tiles_x);
         for (uint32_t t = t0; t < t1; t++, c.next(tiles_x)) body(c.x0(), c.y0());
     });
@@ -125,7 +128,8 @@ template <class R, int A, int F> __global__ void __launch_bounds__(PERSIST_THREA
     SampleGeometry<R> g = make_geometry(a.image, a.size, a.max_iter, a.jcx, a.jcy);
     g.newton = a.newton;
     unsigned long long iters = 0;
-    for_each_tile(a.work.next, a.n_tiles, a.tiles_x, a.tile_chunk, lane, [&](uint32_t x0, uint32_t y0) {
+    constexpr bool even = F >= FRACTAL_NEWTON_WIRED;  // Newton tiles
+    for_each_tile<even>(a.work.next, a.n_tiles, a.tiles_x, a.tile_chunk, lane, [&](uint32_t x0, uint32_t y0) {
         render_main_tile<R, A, F>(g, a.out, a.pitch, a.size, x0, y0, lane, a.max_ss, a.flags, iters);
     });
     add_total(a.total, iters, lane);
@@ -241,7 +245,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS) k_advanced(AdvancedArgs<R> a)
             __syncthreads();
             for_each_claim(claims, 4u, strip);
         } else {
-            for_each_strip(a.m.work.next, a.m.n_tiles, a.m.tile_chunk, lane, strip);
+            for_each_strip<true>(a.m.work.next, a.m.n_tiles, a.m.tile_chunk, lane, strip);
         }
     };
     if (PIECES || al8)
@@ -292,18 +296,28 @@ static inline LaunchShape shape_for(unsigned long long work_warps, int occ, int 
 // binary32 work.
 template <class R, int A> constexpr int main_blocks() { return sizeof(R) == 8 && A != ARITH_FLOATFLOAT ? 2 : 4; }
 
-// And their longest strip.  One warp renders a strip, so its worst case, every
-// step of every sample, is held to a few tiles' share of what the frame gives a
-// warp; single tiles would make the counter the bound of large shallow frames.
-// Default view, us with strips of up to 2 / 4 / 8: 7680x4320, maxIter 16
-// 433 / 407 / 395, 64 509 / 489 / 485, 256 578 / 565 / 571, 1600 832 / 858 / 925
-// (all points outside, any limit: 388 / 357 / 344); 3840x2160, 16 128 / 121 / 119,
-// 64 147 / 146 / 148, 1600 279 / 312 / 346.
+// And their longest strip of tiles.  Single tiles make the counter the bound of
+// shallow frames (0.7 ns a claim), strips lengthen the frame's end: one warp
+// renders a strip, and its worst case, every step of every sample, is about 8 ns
+// a step.  So the tiles past a strip's first may cost a thirtieth of the least
+// such a frame takes, about 0.45 ns (1 + worst / 600) a tile; frames with 32 tiles
+// a warp and more, which a claim a tile could hold up by a quarter of a
+// millisecond, have strips of two at least.  Binary64 tiles take longer than a claim.
+// us with strips of up to 1 / 2 / 4 / 8, default view: 1801x1769 of 1 sample at
+// maxIter 64 83 / 68 / 69 / 69, 250 81 / 71 / 71 / 71, of 5 at 250 124 / 137 / 137 / 137, 1600
+// 282 / 348 / 356 / 356; 3840x2160 of 1 at 64 189 / 143 / 137 / 135, 250 188 / 154 / 154 /
+// 157, 1600 229 / 231 / 252 / 269; 7680x4320 at 64 719 / 501 / 475 / 465, 250 713 / 544 /
+// 521 / 519, 1600 776 / 720 / 728 / 769 (all points outside 717 / 386 / 357 / 344).
+// Longer strips after short tiles: lost wherever the boundary came next (3840x2160 at
+// 1600: 274 us; 1801x1769 in binary64 at 250: 885 -> 1035).
+template <class R>
 static inline uint32_t main_strip(uint32_t n_tiles, int occ, int sms, uint32_t max_iter, float max_ss)
 {
-    const double tiles = (double)n_tiles / ((double)occ * sms * (PERSIST_THREADS / 32));  // a warp's
+    if (sizeof(R) == 8) return 1;
     const double worst = std::max(1.0, (double)max_iter * std::max(1.0, (double)max_ss));
-    return (uint32_t)std::min(8.0, std::max(tiles >= 128.0 ? 4.0 : 2.0, 5.0 * tiles / worst));
+    const double least = 0.45 * n_tiles * (1.0 + worst / 600.0);  // ns
+    const double floor = n_tiles / 32u >= (uint32_t)(occ * sms * (PERSIST_THREADS / 32)) ? 2.0 : 1.0;
+    return (uint32_t)std::min(8.0, std::max(floor, 1.0 + least / 30.0 / (8.0 * worst)));
 }
 
 template <class R, int A, int F> static cudaError_t launch_main_t(const MainArgs<R> &args, int sms, cudaStream_t s)
@@ -313,7 +327,7 @@ template <class R, int A, int F> static cudaError_t launch_main_t(const MainArgs
     const int occ = newton ? fit : std::min(main_blocks<R, A>(), fit);
     MainArgs<R> a = args;
     a.tile_chunk = newton ? tile_chunk_for(a.n_tiles, occ, sms)
-                          : tile_chunk_for(a.n_tiles, occ, sms, main_strip(a.n_tiles, occ, sms, a.max_iter, a.max_ss));
+                          : tile_chunk_for(a.n_tiles, occ, sms, main_strip<R>(a.n_tiles, occ, sms, a.max_iter, a.max_ss));
     const LaunchShape l = shape_for((a.n_tiles + a.tile_chunk - 1) / a.tile_chunk, occ, sms);
     k_main<R, A, F><<<l.blocks, l.threads, 0, s>>>(a);
     return cudaGetLastError();
