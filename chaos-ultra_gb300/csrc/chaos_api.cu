@@ -105,19 +105,27 @@ int device_state(DeviceState **out)
     return CHAOS_OK;
 }
 
-int take_counter(DeviceState *d, cudaStream_t s, WorkCounter *work)
+// sync: the call waits for its launch and gives the slot back itself (give_counter)
+int take_counter(DeviceState *d, cudaStream_t s, bool sync, WorkCounter *work)
 {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     CHAOS_CUDA(cudaStreamIsCapturing(s, &capture), "cudaStreamIsCapturing");
     const uint32_t slot = capture == cudaStreamCaptureStatusNone ? d->ring.take() : SlotRing::NONE;
     if (slot != SlotRing::NONE) {
-        *work = WorkCounter{d->counters + slot, d->counters + 4 * kCounterSlots + slot, d->busy + slot};
+        *work = WorkCounter{d->counters + slot, d->counters + 4 * kCounterSlots + slot,
+                            sync ? nullptr : d->busy + slot};
         return CHAOS_OK;
     }
     const uint32_t k = d->next_zeroed.fetch_add(1, std::memory_order_relaxed) % kCounterSlots;
     *work = WorkCounter{d->counters + kCounterSlots + k, nullptr, nullptr};
     CHAOS_CUDA(cudaMemsetAsync(work->next, 0, sizeof(uint32_t), s), "cudaMemsetAsync(work counter)");
     return CHAOS_OK;
+}
+
+// After a synchronous launch has been waited for without an error
+void give_counter(DeviceState *d, const WorkCounter &work)
+{
+    if (work.done && !work.busy) d->ring.give((uint32_t)(work.next - d->counters));
 }
 
 // The status word that goes with a counter (a launch with a time limit
@@ -155,6 +163,13 @@ int finish(cudaError_t launch, cudaStream_t s, bool sync)
     if (launch != cudaSuccess) return cuda_fail(launch, "kernel launch");
     if (sync) CHAOS_CUDA(cudaStreamSynchronize(s), "cudaStreamSynchronize");
     return CHAOS_OK;
+}
+
+int finish_work(DeviceState *d, const WorkCounter &work, cudaError_t launch, cudaStream_t s, bool sync)
+{
+    const int rc = finish(launch, s, sync);
+    if (sync && rc == CHAOS_OK) give_counter(d, work);
+    return rc;
 }
 
 template <class R> bool finite4(const R r[4])
@@ -347,13 +362,19 @@ void api_prefault(void *p, size_t bytes)
     if (at.type == cudaMemoryTypeUnregistered) populate_pages(p, bytes);
 }
 
-int api_device_counter(cudaStream_t s, WorkCounter *work, int *sms)
+int api_device_counter(cudaStream_t s, bool sync, WorkCounter *work, int *sms)
 {
     DeviceState *d;
     int rc = device_state(&d);
     if (rc) return rc;
     *sms = d->sms;
-    return take_counter(d, s, work);
+    return take_counter(d, s, sync, work);
+}
+
+void api_device_counter_done(const WorkCounter &work)
+{
+    DeviceState *d;
+    if (device_state(&d) == CHAOS_OK) give_counter(d, work);
 }
 
 int api_device_status(const WorkCounter &work, cudaStream_t s, uint32_t **status)
@@ -565,8 +586,8 @@ static int render_main(chaos_module *m, chaos_pixel_info *out, long pitch, uint3
     a.newton = m->newton;
     a.tiles_x = (w + 7u) / 8u;
     a.n_tiles = a.tiles_x * ((h + 3u) / 4u);
-    if ((rc = take_counter(d, s, &a.work))) return rc;
-    return finish(launch_main<R>(a, arith_of(arith), m->fractal, d->sms, s), s, sync);
+    if ((rc = take_counter(d, s, sync, &a.work))) return rc;
+    return finish_work(d, a.work, launch_main<R>(a, arith_of(arith), m->fractal, d->sms, s), s, sync);
 }
 
 template <class R>
@@ -607,8 +628,8 @@ static int render_advanced(chaos_module *m, chaos_pixel_info *out, long pitch, u
     a.in = in;
     a.in_pitch = in_pitch;
     a.focus = UInt2{fx, fy};
-    if ((rc = take_counter(d, s, &a.m.work))) return rc;
-    return finish(launch_advanced<R>(a, arith_of(arith), m->fractal, d->sms, s), s, sync);
+    if ((rc = take_counter(d, s, sync, &a.m.work))) return rc;
+    return finish_work(d, a.m.work, launch_advanced<R>(a, arith_of(arith), m->fractal, d->sms, s), s, sync);
 }
 
 int chaos_render_main_f32(chaos_module *m, chaos_pixel_info *out, long pitch, uint32_t width, uint32_t height,
@@ -763,11 +784,14 @@ static int frame_impl(const chaos_frame_desc *dsc, const chaos_frame_out *o, cud
     const bool own_status = a.budget_ns && !a.status;
     if (own_status && !sync && !status_used)
         return fail(CHAOS_ERR_INVALID_ARGUMENT, "a time limit on an unsynchronised frame needs out->status");
-    if ((rc = take_counter(d, s, &a.work))) return rc;
+    if ((rc = take_counter(d, s, sync, &a.work))) return rc;
     if (own_status && (rc = take_status(d, a.work, s, &a.status))) return rc;
     if (status_used) *status_used = a.budget_ns ? a.status : nullptr;
     if ((rc = finish(launch_frame<R>(a, arith_of(dsc->arith), (int)dsc->fractal, d->sms, s), s, sync))) return rc;
-    return sync && a.budget_ns ? read_status(a.status, s, dsc->time_limit_s) : CHAOS_OK;
+    if (!sync) return CHAOS_OK;
+    if (a.budget_ns) rc = read_status(a.status, s, dsc->time_limit_s);
+    give_counter(d, a.work);  // (after its status word has been read)
+    return rc;
 }
 
 static int frame_entry(const chaos_frame_desc *dsc, const chaos_frame_out *o, cudaStream_t s, bool sync,

@@ -17,9 +17,10 @@
 namespace chaos {
 
 // A launch's work counter (`next`; zero when the launch starts) and its slot's
-// other words, null where the caller or a memset before the launch zeroes the
-// counter: the number of blocks that have ended (zero between launches) and the
-// host's word that says the slot is taken (chaos_slots.h).
+// other words: the number of blocks that have ended (zero between launches; null
+// where the caller or a memset before the launch zeroes the counter) and the
+// host's word that says the slot is taken (chaos_slots.h; null where the host
+// gives the slot back).
 struct WorkCounter {
     uint32_t *next, *done, *busy;
 };
@@ -39,6 +40,7 @@ __device__ __forceinline__ void leave_counter(const WorkCounter &w, uint32_t *re
     if (atomicAdd(w.done, 1u) + 1u != gridDim.x) return;
     *w.next = 0u;
     *w.done = 0u;
+    if (!w.busy) return;
     __threadfence_system();
     *(volatile uint32_t *)w.busy = 0u;
 }

@@ -57,7 +57,8 @@
 namespace chaos {
 
 int api_fail(int code, const char *fmt, ...);  // chaos_api.cu
-int api_device_counter(cudaStream_t s, WorkCounter *work, int *sms);
+int api_device_counter(cudaStream_t s, bool sync, WorkCounter *work, int *sms);
+void api_device_counter_done(const WorkCounter &work);
 int api_device_status(const WorkCounter &work, cudaStream_t s, uint32_t **status);
 bool api_budget(double seconds, unsigned long long *ns);
 int api_read_status(const uint32_t *status, cudaStream_t s, double seconds);
@@ -1102,7 +1103,7 @@ static int perturb_impl(const chaos_frame_desc *d, const chaos_orbit *orb, const
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     } else {
-        int rc = api_device_counter(s, &a.work, &sms);
+        int rc = api_device_counter(s, sync, &a.work, &sms);
         if (rc) return rc;
     }
     if (own_status) {
@@ -1119,7 +1120,9 @@ static int perturb_impl(const chaos_frame_desc *d, const chaos_orbit *orb, const
     if (sync) {
         e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return api_fail(CHAOS_ERR_CUDA, "cudaStreamSynchronize: %s", cudaGetErrorString(e));
-        if (a.budget_ns) return api_read_status(a.status, s, d->time_limit_s);
+        const int rc = a.budget_ns ? api_read_status(a.status, s, d->time_limit_s) : CHAOS_OK;
+        if (!counter) api_device_counter_done(a.work);  // (after its status word has been read)
+        return rc;
     }
     return CHAOS_OK;
 }

@@ -7,7 +7,9 @@
 // warp, so no event or query is needed, and a stream capture elsewhere is not
 // disturbed.  Going by the order of the launches instead would hand the slot of
 // a frame of seconds to another stream's preview after 4096 previews (80 ms).
-// A launch that never ran keeps its slot.
+// A launch that the caller's own call waits for is given back here instead: the
+// write to the host is the end of such a launch (200x110 pixels: 18.1 us with it,
+// 17.2 without).  A launch that never ran keeps its slot.
 #pragma once
 
 #include <atomic>
@@ -40,6 +42,9 @@ public:
         }
         return NONE;
     }
+
+    // A slot whose launch has been waited for.
+    void give(uint32_t slot) { __atomic_store_n(busy_ + slot, 0u, __ATOMIC_RELEASE); }
 
 private:
     uint32_t *busy_ = nullptr;
