@@ -88,9 +88,13 @@ int device_state(DeviceState **out)
         constexpr size_t words = 5 * kCounterSlots;
         cudaError_t e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
         if (e == cudaSuccess) e = cudaMalloc(&d.counters, words * sizeof(uint32_t));
-        // (on the legacy stream, and waited for: the first launch may be on any other)
-        if (e == cudaSuccess) e = cudaMemset(d.counters, 0, words * sizeof(uint32_t));
-        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+        // (waited for: the first launch may be on any stream; and not on the legacy one,
+        // which may not be used while the caller records one that orders itself with it)
+        cudaStream_t own = nullptr;
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaMemsetAsync(d.counters, 0, words * sizeof(uint32_t), own);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+        if (own) cudaStreamDestroy(own);
         uint32_t *busy = nullptr;
         if (e == cudaSuccess) e = cudaHostAlloc(&busy, kCounterSlots * sizeof(uint32_t), cudaHostAllocMapped);
         if (e == cudaSuccess) {
