@@ -155,7 +155,14 @@ constexpr uint32_t PIECE_TILES = 4 * PERSIST_THREADS / 32;  // a group of four f
 // tile (l >> 2) & 3) and taken by shuffles.  The filtered (value, weight)
 // pairs (the weight -1 where the origin is out of range) go to the warp's
 // `stage` (4 x 32 pairs of shared memory), from which each tile is finished
-// in its own 8x4 lane layout (votes, samples, record).
+// in its own 8x4 lane layout (votes, samples, record): the group's tiles that
+// only reuse first, then the others, in a loop of their own with one copy of
+// the sampling code.  Sampled within the loop of all four, which is unrolled,
+// it was 200 KB of code (790 KB in binary64; 74 and 229 so), and the warps of a
+// frame that samples its borders waited for instructions (1.7 of every 13 cycles
+// a warp is resident for an instruction; 0.8 with less code): zooming out at
+// 7000x4000, span 3, maxIter 133, 2 samples 252 -> 209 us, 4681x4384 184 -> 164,
+// 5199x4054 of the antenna, maxIter 274, 435 -> 382.
 template <class R, int A, int F, bool AL8>
 __device__ __forceinline__ void advanced_strip(const AdvancedArgs<R> &a, const SampleGeometry<R> &g, uint32_t lane,
                                                float2 *stage, uint32_t t0, uint32_t t1, unsigned long long &iters)
@@ -195,25 +202,37 @@ __device__ __forceinline__ void advanced_strip(const AdvancedArgs<R> &a, const S
             }
             __syncwarp();
         }
-        for (uint32_t k = 0; k < ng; k++, cur.next(tiles_x)) {
-            const uint32_t x0 = cur.x0(), y0 = cur.y0();
+        // the tiles whose pixels all reuse and take no new samples: the record is
+        // (value, weight, isReused = 1, 0), as the full path stores it
+        TileCursor at = cur;
+        uint32_t rest = 0;  // the others
+        for (uint32_t k = 0; k < ng; k++, at.next(tiles_x)) {
+            const uint32_t x0 = at.x0(), y0 = at.y0();
             const UInt2 p = tile_pixel(x0, y0, lane);
             const bool valid = p.x < a.m.size.x && p.y < a.m.size.y;
             const float2 vw = reuse ? stage[32u * row + 8u * k + col] : make_float2(0.f, 0.f);
             const bool reusing = valid && reuse && !(vw.y < 0.1f);
             if ((!fov || clear_of_fovea(a.focus, x0, y0)) && __all_sync(FULL, reusing || !valid)) {
-                // every pixel reuses and none takes new samples: the record is
-                // (value, weight, isReused = 1, 0), as the full path stores it
                 if (valid) {
                     PixelInfo rec = make_pixel(vw.x, vw.y);
                     rec.is_reused = 1;
                     store_pixel_streaming(pixel_ptr(a.m.out, a.m.pitch, p.x, p.y), rec);
                 }
-                continue;
+            } else {
+                rest |= 1u << k;
             }
-            finish_advanced_tile<R, A, F>(g, a.m.out, a.m.pitch, a.m.size, a.focus, x0, y0, lane, a.m.max_ss,
-                                          a.m.flags, reusing, vw.x, vw.y, iters);
         }
+        while (rest) {
+            const uint32_t k = __ffs(rest) - 1u;
+            rest &= rest - 1u;
+            const TileCursor c = cur.plus(k, tiles_x);
+            const UInt2 p = tile_pixel(c.x0(), c.y0(), lane);
+            const bool valid = p.x < a.m.size.x && p.y < a.m.size.y;
+            const float2 vw = reuse ? stage[32u * row + 8u * k + col] : make_float2(0.f, 0.f);
+            finish_advanced_tile<R, A, F>(g, a.m.out, a.m.pitch, a.m.size, a.focus, c.x0(), c.y0(), lane, a.m.max_ss,
+                                          a.m.flags, valid && reuse && !(vw.y < 0.1f), vw.x, vw.y, iters);
+        }
+        cur = at;
         __syncwarp();
     }
 }
