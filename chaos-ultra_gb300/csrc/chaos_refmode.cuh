@@ -34,24 +34,33 @@ __device__ __forceinline__ void add_total(unsigned long long *total, unsigned lo
 // before it is rendered.  Where a tile may run for long, the strip that its warp
 // holds already would wait as long, so strips are claimed when needed
 // (1801x1769, maxIter 1600, 5 samples, strips of two: 413 us ahead, 348).
-template <bool AHEAD, class Body>
+// SPREAD: the warps' first strips go out without a claim, neighbouring ones to
+// different SMs.  Claimed, a block's warps take neighbouring tiles: the sampled
+// border at the top of a binary64 zoom-out was on a third of the SMs, eight warps
+// to a binary64 pipe (966x515, maxIter 300, 2 samples 385 -> 306 us; in binary32,
+// where the rows' reads come from the L2 together, 5199x4054 382 -> 403).
+template <bool AHEAD, bool SPREAD, class Body>
 __device__ __forceinline__ void for_each_strip(uint32_t *counter, uint32_t n_tiles, uint32_t max_chunk, uint32_t lane,
                                                Body body)
 {
-    const uint32_t share = 4u * gridDim.x * (blockDim.x >> 5);
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5), share = 4u * warps;
     auto size_after = [&](uint32_t at) -> uint32_t {
         const uint32_t c = (at < n_tiles ? n_tiles - at : 0u) / share;
         return c < 1u ? 1u : c > max_chunk ? max_chunk : c;
     };
     uint32_t size = size_after(0u), claim = 0;
-    if (lane == 0) claim = atomicAdd(counter, size);
+    const uint32_t base = SPREAD ? warps * size : 0u;  // claims count from here
+    if (SPREAD)
+        claim = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * size;
+    else if (lane == 0)
+        claim = atomicAdd(counter, size);
     uint32_t t0 = __shfl_sync(FULL, claim, 0);
     while (t0 < n_tiles) {
         const uint32_t t1 = min(t0 + size, n_tiles), next = size_after(t1);
         const bool ahead = AHEAD && size > 1u;
-        if (ahead && lane == 0) claim = atomicAdd(counter, next);
+        if (ahead && lane == 0) claim = base + atomicAdd(counter, next);
         body(t0, t1);
-        if (!ahead && lane == 0) claim = atomicAdd(counter, next);
+        if (!ahead && lane == 0) claim = base + atomicAdd(counter, next);
         t0 = __shfl_sync(FULL, claim, 0);
         size = next;
     }
@@ -102,7 +111,7 @@ template <bool AHEAD, class Body>
 __device__ __forceinline__ void for_each_tile(uint32_t *counter, uint32_t n_tiles, uint32_t tiles_x, uint32_t chunk,
                                               uint32_t lane, Body body)
 {
-    for_each_strip<AHEAD>(counter, n_tiles, chunk, lane, [&](uint32_t t0, uint32_t t1) {
+    for_each_strip<AHEAD, false>(counter, n_tiles, chunk, lane, [&](uint32_t t0, uint32_t t1) {
         TileCursor c(t0, tiles_x);
         for (uint32_t t = t0; t < t1; t++, c.next(tiles_x)) body(c.x0(), c.y0());
     });
@@ -264,7 +273,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS) k_advanced(AdvancedArgs<R> a)
             __syncthreads();
             for_each_claim(claims, 4u, strip);
         } else {
-            for_each_strip<true>(a.m.work.next, a.m.n_tiles, a.m.tile_chunk, lane, strip);
+            for_each_strip<true, sizeof(R) == 8>(a.m.work.next, a.m.n_tiles, a.m.tile_chunk, lane, strip);
         }
     };
     if (PIECES || al8)
