@@ -374,7 +374,7 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
 // that go on (samples close to the boundary, interiors of the smaller
 // components) go on for hundreds.  Mixed in one warp, each long orbit held its
 // 31 neighbours to a round of 64 steps.  So a warp takes fresh pixels 32 at a
-// time and gives every sample up to FRESH_STEPS steps; samples still running
+// time and gives every sample up to `fresh_steps` steps; samples still running
 // then wait in the warp's queue in shared memory, and when the queue holds a
 // warp's worth they run by themselves in rounds of 64 steps, lanes that end
 // refilled from the queue, until fewer than REQUEUE lanes are left.  When the
@@ -395,7 +395,14 @@ template <int A, int F> __global__ void __launch_bounds__(PERSIST_THREADS) k_fra
 // the long orbits, 51 with ended samples written several at a time, 46 with
 // packing and the skew (FRESH_STEPS 16: 49; REQUEUE 12: 49).  256x144 pixels,
 // maxIter 500: 20.6 -> 15.
-constexpr int FRESH_STEPS = 32;
+//
+// Samples that the iteration limit ends soon are not worth a queue: up to
+// FRESH_ALL steps a batch runs to the limit as it is, and up to FRESH_ALL_SMALL
+// where no warp has a second batch.  us with per-lane refill / 32 fresh steps /
+// all: Julia set, 260x240 of 4 samples, maxIter 50 23 / 38 / 22, 134 46 / 50 / 28;
+// 1500x1000 of 1 at 50 47 / 57 / 41, 200 71 / 72 / 69, 256 73 / 74 / 79; -1.25, span
+// 0.2, 370x280 at 500 41 / 40 / 34, 2400x1700 at 200 374 / 190 / 205.
+constexpr uint32_t FRESH_STEPS = 32, FRESH_ALL = 200, FRESH_ALL_SMALL = 512;
 constexpr int LONG_STEPS = 64;
 constexpr uint32_t REQUEUE = 24;
 constexpr int MAX_EPOCH = 16;         // rounds between packings, at most
@@ -405,7 +412,8 @@ constexpr uint32_t QUEUE = 64;  // entries per warp: at most 31 waiting and 32 f
 template <bool MULTI> constexpr int frame32_threads() { return MULTI ? 256 : 512; }
 
 template <int A, int F, bool MULTI>
-__global__ void __launch_bounds__(frame32_threads<MULTI>()) k_frame32(FrameArgs<float> a, uint32_t fixed_rounds)
+__global__ void __launch_bounds__(frame32_threads<MULTI>())
+k_frame32(FrameArgs<float> a, uint32_t fixed_rounds, uint32_t fresh_steps)
 {
     constexpr int WORDS = MULTI ? 12 : 6, WARPS = frame32_threads<MULTI>() / 32;
     __shared__ uint32_t s_pal[PALETTE_SMEM];
@@ -620,7 +628,7 @@ __global__ void __launch_bounds__(frame32_threads<MULTI>()) k_frame32(FrameArgs<
                 if (live) {
                     bool ended = start();
                     if (!ended) {
-                        const uint32_t end = a.max_iter - i > (uint32_t)FRESH_STEPS ? i + FRESH_STEPS : a.max_iter;
+                        const uint32_t end = a.max_iter - i > fresh_steps ? i + fresh_steps : a.max_iter;
                         tested_steps<float, A>(x, y, cx, cy, i, end, r2);
                         ended = !(r2 < 4.f) || i == a.max_iter;
                     }
@@ -861,7 +869,8 @@ template <int A, int F, bool MULTI> static cudaError_t launch_frame32_t(const Fr
     const unsigned long long n_warps = (unsigned long long)grid * warps;
     uint32_t fixed = (uint32_t)(batches * 5ull / 8ull / n_warps);  // rounds of fixed batches
     if (fixed < 1) fixed = 1;
-    k_frame32<A, F, MULTI><<<grid, threads, 0, s>>>(a, fixed);
+    const uint32_t all = batches <= n_warps ? FRESH_ALL_SMALL : FRESH_ALL;
+    k_frame32<A, F, MULTI><<<grid, threads, 0, s>>>(a, fixed, a.max_iter <= all ? all : FRESH_STEPS);
     return cudaGetLastError();
 }
 template <int A, int F> static cudaError_t launch_frame32(const FrameArgs<float> &a, int sms, cudaStream_t s)
