@@ -252,7 +252,7 @@ class Batch:
         return t.value
 
     def read_cycle_skipped(self):
-        """Iterations of the last launch proven interior by a repeated state and not run."""
+        """Iterations of the last launch proven interior (by the point or a repeated state) and not run."""
         t = C.c_ulonglong()
         check(lib().chaos_batch_read_cycle_skipped(self.handle, C.byref(t)))
         return t.value

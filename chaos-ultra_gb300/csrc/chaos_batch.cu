@@ -47,7 +47,7 @@ struct BatchArgs {
     uint32_t n_vp, n_jobs;
     uint32_t chunk;  // consecutive jobs a lane claims per work-counter update
     uint32_t *counter;
-    unsigned long long *total;  // [0] pixel-iterations, [1] iterations proven interior by a repeated state, not run
+    unsigned long long *total;  // [0] pixel-iterations, [1] iterations proven interior (by c or a repeated state), not run
     const uint32_t *palette;
     uint32_t palette_len;
     uint32_t interior_rgba;

@@ -66,7 +66,7 @@ template <class R> struct FrameArgs {
     uint32_t interior_rgba;
     unsigned long long *total;
     WorkCounter work;
-    unsigned long long *skipped;  // optional: iterations of interior samples proven by a repeated state, not run
+    unsigned long long *skipped;  // optional: iterations of interior samples proven such (by their c or a repeated state), not run
     unsigned long long budget_ns; // 0, or the run time after which warps stop (RUN_STATUS_TIMEOUT into *status)
     uint32_t *status;
 };

@@ -296,8 +296,10 @@ struct LaunchShape {
 };
 
 // The launch for work that `work_warps` warps share, up to `occ` blocks an SM.
-// Work that fits goes out in as few blocks an SM as hold it, sized so that every
-// SM gets the same number of warps: full blocks put the 437 tiles of a 150x90
+// Work that fits goes out in blocks sized for the busiest SM: it gets no more than
+// an even share, rounded up to whole warps of each of its blocks (just above a
+// multiple of the SMs others get fewer: 153 tiles are 77 blocks of two warps).
+// Full blocks put the 437 tiles of a 150x90
 // frame on 55 of the 152 SMs and a 300x200 frame's 1900 on 86 SMs twice and on
 // 66 once.  Seahorse valley, maxIter 3500, 2 samples in binary64, whose warps
 // queue for their SM's pipe: 2823 / 1767 us and 5543 /
