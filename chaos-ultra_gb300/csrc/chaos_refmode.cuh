@@ -56,13 +56,18 @@ __device__ __forceinline__ void for_each_strip(uint32_t *counter, uint32_t n_til
         claim = atomicAdd(counter, size);
     uint32_t t0 = __shfl_sync(FULL, claim, 0);
     while (t0 < n_tiles) {
-        const uint32_t t1 = min(t0 + size, n_tiles), next = size_after(t1);
+        const uint32_t t1 = min(t0 + size, n_tiles);
         const bool ahead = AHEAD && size > 1u;
-        if (ahead && lane == 0) claim = base + atomicAdd(counter, next);
+        if (ahead) {
+            size = size_after(t1);
+            if (lane == 0) claim = base + atomicAdd(counter, size);
+        }
         body(t0, t1);
-        if (!ahead && lane == 0) claim = base + atomicAdd(counter, next);
+        if (!ahead) {
+            size = size_after(t1);
+            if (lane == 0) claim = base + atomicAdd(counter, size);
+        }
         t0 = __shfl_sync(FULL, claim, 0);
-        size = next;
     }
 }
 
